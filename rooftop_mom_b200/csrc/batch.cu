@@ -56,7 +56,7 @@ int BatchOp::apply(const void* x, void* y, int nrhs, cudaStream_t s, SkipFlags s
             return fail(RTM_ERR_ARG, "the plate batch was not reserved");
         RTM_TRY(apply_plate_batch(plates, descs.ptr, stride, work.ptr, fault, x, y, s, skip));
     } else if (fused_bj) {
-        RTM_TRY(apply_block_jacobi_batch(descs.as<BjEntry>(), (int)ops.size(), bj_blocks, bj_S, precision, x, y, stride,
+        RTM_TRY(apply_block_jacobi_batch(descs.as<BjShape>(), (int)ops.size(), bj_blocks, bj_S, precision, x, y, stride,
                                          s, skip));
     } else {
         const size_t elem = precision == RTM_FP64 ? sizeof(double2) : sizeof(float2);
@@ -111,14 +111,14 @@ std::unique_ptr<BatchOp> make_batch(const std::vector<LinearOp*>& ops, int64_t s
         } else {
             b->plates.clear();
         }
-        std::vector<BjEntry> bj(ops.size());
+        std::vector<BjShape> bj(ops.size());
         bool all_bj = !b->fused;
         for (size_t k = 0; k < ops.size() && all_bj; ++k)
             all_bj = block_jacobi_entry(ops[k], &bj[k]) && bj[k].S == bj[0].S;
         if (all_bj) {
-            for (const BjEntry& e : bj) b->bj_blocks = std::max(b->bj_blocks, e.nblocks);
+            for (const BjShape& e : bj) b->bj_blocks = std::max(b->bj_blocks, e.nbx * e.nby);
             b->bj_S = bj[0].S;
-            if ((*status = b->descs.alloc(sizeof(BjEntry) * bj.size())) != RTM_OK) return nullptr;
+            if ((*status = b->descs.alloc(sizeof(BjShape) * bj.size())) != RTM_OK) return nullptr;
             if ((*status = check_cuda(cudaMemcpyAsync(b->descs.ptr, bj.data(), b->descs.bytes, cudaMemcpyHostToDevice, s),
                                       "cudaMemcpyAsync")) != RTM_OK)
                 return nullptr;

@@ -58,35 +58,28 @@ std::unique_ptr<LinearOp> make_dense_op(const double2* device_matrix, int64_t n,
 }
 
 // ---------------------------------------------------------------------------------------------
+// Block-Jacobi. A block's matrix depends on the offsets between its rooftops alone, and only the last block
+// column and the last block row lack rooftops (their last faces are no first faces), so a plate has four
+// distinct block matrices at most: class (last column) + 2 (last row). Four inverses are formed and stored; the
+// apply reads them from the caches instead of one inverse per block (the 256 x 256 plate's 16.8 MB).
 constexpr int kMaxBlockUnknowns = 16;
+constexpr int kBlockClasses = 4;
 
-struct BjArgs {
-    int cx, cy, bx, by, nbx, nby;
-    double a, b;
-    const double2* E;
-    const double2* XX;
-    const double2* YY;
-    int64_t nx_roof;             // x-directed rooftops (offset of the y-directed ones)
-    int* counts;                 // [blocks]
-    int64_t* index;              // [blocks][kMaxBlockUnknowns]
-    double2* inv;                // [blocks][kMaxBlockUnknowns^2], row-major
-    int* singular;
-};
-
-__device__ double2 green_entry(const BjArgs& g, int dp, int ip, int jp, int dq, int iq, int jq) {
+__device__ double2 green_entry(const BjShape& g, const double2* E, const double2* XX, const double2* YY, double a,
+                               double b, int dp, int ip, int jp, int dq, int iq, int jq) {
     double re = 0, im = 0;
     if (dp == dq) {
         const int dx = abs(ip - iq), dy = abs(jp - jq);
-        const double2 m = dp == 0 ? g.XX[dx + (int64_t)(g.cx - 1) * dy] : g.YY[dx + (int64_t)g.cx * dy];
+        const double2 m = dp == 0 ? XX[dx + (int64_t)(g.cx - 1) * dy] : YY[dx + (int64_t)g.cx * dy];
         re = m.x;
         im = m.y;
     }
-    const double hp = dp == 0 ? g.a : g.b, hq = dq == 0 ? g.a : g.b;
+    const double hp = dp == 0 ? a : b, hq = dq == 0 ? a : b;
     for (int s = 0; s < 2; ++s) {
         const int fi = ip + (s && dp == 0), fj = jp + (s && dp == 1);
         for (int t = 0; t < 2; ++t) {
             const int gi = iq + (t && dq == 0), gj = jq + (t && dq == 1);
-            const double2 e = g.E[abs(fi - gi) + (int64_t)g.cx * abs(fj - gj)];
+            const double2 e = E[abs(fi - gi) + (int64_t)g.cx * abs(fj - gj)];
             const double w = ((s == t) ? 1.0 : -1.0) / (hp * hq);
             re -= w * e.x;
             im -= w * e.y;
@@ -95,97 +88,124 @@ __device__ double2 green_entry(const BjArgs& g, int dp, int ip, int jp, int dq, 
     return make_double2(re, im);
 }
 
-// One thread per block: gather its rooftops, form the block of the Green's matrix, invert it by
-// Gauss-Jordan elimination with partial pivoting.
-__global__ void k_bj_build(const BjArgs g) {
-    const int blk = blockIdx.x * blockDim.x + threadIdx.x;
-    if (blk >= g.nbx * g.nby) return;
-    const int I = blk % g.nbx, J = blk / g.nbx;
-    int dir[kMaxBlockUnknowns], fi[kMaxBlockUnknowns], fj[kMaxBlockUnknowns];
-    int64_t* idx = g.index + (int64_t)blk * kMaxBlockUnknowns;
-    int cnt = 0;
-    for (int d = 0; d < 2; ++d)
-        for (int j = J * g.by; j < min((J + 1) * g.by, g.cy); ++j)
-            for (int i = I * g.bx; i < min((I + 1) * g.bx, g.cx); ++i) {
-                if (d == 0 && i > g.cx - 2) continue;
-                if (d == 1 && j > g.cy - 2) continue;
-                dir[cnt] = d;
-                fi[cnt] = i;
-                fj[cnt] = j;
-                idx[cnt] = d == 0 ? i + (int64_t)(g.cx - 1) * j : g.nx_roof + i + (int64_t)g.cx * j;
-                ++cnt;
-            }
-    g.counts[blk] = cnt;
-    double2 A[kMaxBlockUnknowns][kMaxBlockUnknowns], B[kMaxBlockUnknowns][kMaxBlockUnknowns];
-    for (int r = 0; r < cnt; ++r)
-        for (int c = 0; c < cnt; ++c) {
-            A[r][c] = green_entry(g, dir[r], fi[r], fj[r], dir[c], fi[c], fj[c]);
-            B[r][c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
-        }
-    for (int col = 0; col < cnt; ++col) {
-        int piv = col;
-        double best = -1;
-        for (int r = col; r < cnt; ++r) {
-            const double v = A[r][col].x * A[r][col].x + A[r][col].y * A[r][col].y;
-            if (v > best) { best = v; piv = r; }
-        }
-        if (!(best > 0)) { atomicExch(g.singular, 1); return; }
-        if (piv != col)
-            for (int c = 0; c < cnt; ++c) {
-                double2 t = A[col][c]; A[col][c] = A[piv][c]; A[piv][c] = t;
-                t = B[col][c]; B[col][c] = B[piv][c]; B[piv][c] = t;
-            }
-        const double2 p = A[col][col];
-        const double d = p.x * p.x + p.y * p.y;
-        const double2 inv = make_double2(p.x / d, -p.y / d);
-        for (int c = 0; c < cnt; ++c) { A[col][c] = cmul(A[col][c], inv); B[col][c] = cmul(B[col][c], inv); }
-        for (int r = 0; r < cnt; ++r) {
-            if (r == col) continue;
-            const double2 f = A[r][col];
-            for (int c = 0; c < cnt; ++c) {
-                A[r][c] = csub(A[r][c], cmul(f, A[col][c]));
-                B[r][c] = csub(B[r][c], cmul(f, B[col][c]));
-            }
-        }
+// The unknowns of a block with wx x wy faces, rx of its faces with an x-directed rooftop per row and ry rows of
+// faces with y-directed ones: x-directed rooftops first, i fastest.
+struct BlockLayout {
+    int wx, wy, rx, ry;
+    __host__ __device__ int count() const { return rx * wy + wx * ry; }
+    // direction and first face (within the block) of unknown r < count()
+    __device__ void unknown(int r, int& dir, int& i, int& j) const {
+        dir = r >= rx * wy;
+        const int q = dir ? r - rx * wy : r, w = dir ? wx : rx;
+        j = q / w;
+        i = q - j * w;
     }
-    double2* out = g.inv + (int64_t)blk * kMaxBlockUnknowns * kMaxBlockUnknowns;
-    for (int r = 0; r < cnt; ++r)
-        for (int c = 0; c < cnt; ++c) out[r * kMaxBlockUnknowns + c] = B[r][c];
+};
+// Layout of the blocks in column class lx and row class ly (1: the last one).
+__host__ __device__ inline BlockLayout block_layout(const BjShape& g, int lx, int ly) {
+    BlockLayout l;
+    l.wx = lx ? g.cx - (g.nbx - 1) * g.bx : g.bx;
+    l.wy = ly ? g.cy - (g.nby - 1) * g.by : g.by;
+    l.rx = lx ? l.wx - 1 : g.bx;
+    l.ry = ly ? l.wy - 1 : g.by;
+    return l;
 }
 
-// The inverses packed to S = 2 bx by unknowns a block, column-major inside the block (entry (r, c) at
-// blk S^2 + c S + r), so the S threads of a block read S consecutive entries per column.
+// One CTA per class, a thread per entry of [A | B]: forms the block of the Green's matrix and inverts it by
+// Gauss-Jordan elimination with partial pivoting in shared memory; a chain of at most 16 columns, latency bound
+// (one thread per block of the plate had taken 175 us on the 256 x 256 plate). Writes the inverse packed
+// column-major with S = 2 bx by unknowns (entry (r, c) at class S^2 + c S + r).
+constexpr int kBuildThreads = kMaxBlockUnknowns * kMaxBlockUnknowns;
 template <typename T2>
-__global__ void k_bj_pack(int nblocks, int S, const double2* __restrict__ inv64, const int64_t* __restrict__ index,
-                          T2* __restrict__ out, int64_t* __restrict__ packed_index) {
-    const int64_t total = (int64_t)nblocks * S * S;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t blk = t / ((int64_t)S * S);
-        const int e = (int)(t - blk * S * S), c = e / S, r = e % S;
-        const double2 v = inv64[(blk * kMaxBlockUnknowns + r) * kMaxBlockUnknowns + c];
-        out[t] = cmake<T2>(v.x, v.y);
-        if (e < S) packed_index[blk * S + e] = index[blk * kMaxBlockUnknowns + e];
+__global__ void __launch_bounds__(kBuildThreads) k_bj_build(const BjShape g, const double2* __restrict__ E,
+                                                            const double2* __restrict__ XX,
+                                                            const double2* __restrict__ YY, double a, double b,
+                                                            T2* __restrict__ out, int* __restrict__ singular) {
+    __shared__ double2 A[kMaxBlockUnknowns][kMaxBlockUnknowns + 1], B[kMaxBlockUnknowns][kMaxBlockUnknowns + 1];
+    __shared__ int pivot;
+    const int lx = blockIdx.x & 1, ly = blockIdx.x >> 1;
+    T2* dst = out + (int64_t)blockIdx.x * g.S * g.S;
+    const int r = threadIdx.x % kMaxBlockUnknowns, c = threadIdx.x / kMaxBlockUnknowns;
+    const bool present = (lx || g.nbx > 1) && (ly || g.nby > 1);  // some block of the plate is of this class
+    const BlockLayout l = block_layout(g, lx, ly);
+    const int cnt = present ? l.count() : 0;
+    if (r < g.S && c < g.S) dst[c * g.S + r] = czero<T2>();
+    const bool in = r < cnt && c < cnt;
+    if (in) {
+        int dp, ip, jp, dq, iq, jq;
+        l.unknown(r, dp, ip, jp);
+        l.unknown(c, dq, iq, jq);
+        A[r][c] = green_entry(g, E, XX, YY, a, b, dp, ip, jp, dq, iq, jq);
+        B[r][c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
     }
+    __syncthreads();
+    for (int col = 0; col < cnt; ++col) {
+        if (threadIdx.x == 0) {
+            int piv = col;
+            double best = -1;
+            for (int q = col; q < cnt; ++q) {
+                const double v = A[q][col].x * A[q][col].x + A[q][col].y * A[q][col].y;
+                if (v > best) { best = v; piv = q; }
+            }
+            pivot = best > 0 ? piv : -1;
+        }
+        __syncthreads();
+        const int piv = pivot;
+        if (piv < 0) {
+            if (threadIdx.x == 0) atomicExch(singular, 1);
+            return;
+        }
+        // row `col` after the exchange and its scaling, and every row's factor, read before anything is written
+        double2 pa, pb, f, own_a, own_b;
+        if (in) {
+            const double2 p = A[piv][col];
+            const double d = p.x * p.x + p.y * p.y;
+            const double2 inv = make_double2(p.x / d, -p.y / d);
+            pa = cmul(A[piv][c], inv);
+            pb = cmul(B[piv][c], inv);
+            const int src = r == piv ? col : r;  // the row that stands at r after the exchange
+            f = A[src][col];
+            own_a = A[src][c];
+            own_b = B[src][c];
+        }
+        __syncthreads();
+        if (in) {
+            A[r][c] = r == col ? pa : csub(own_a, cmul(f, pa));
+            B[r][c] = r == col ? pb : csub(own_b, cmul(f, pb));
+        }
+        __syncthreads();
+    }
+    if (in) dst[c * g.S + r] = cmake<T2>(B[r][c].x, B[r][c].y);
 }
 
 // y(idx_r) = sum_c inv(r, c) x(idx_c) over the block's unknowns, one thread per (block, row). Where S divides
 // the warp (blocks of 1, 2, 4, 8 or 16 unknowns, 2 x 2 faces among them), the S threads of a block each gather
-// their own x(idx_r) and pass it to the others by warp shuffles, so a thread issues one index and one vector
-// load instead of S of each; the sum runs over c in the same order either way.
+// their own x(idx_r) and pass it to the others by warp shuffles, so a thread issues one vector load instead of S;
+// the sum runs over c in the same order either way. Bound: the vectors (read and written once); the inverses
+// stay in L1. The 256 x 256 plate, FP64: 7.2 us with an inverse and an index list per block.
 template <typename T2, int SC>  // SC: S as a compile-time constant (the loops unroll), or 0
-__device__ __forceinline__ void bj_rows(int nblocks, int S_, const int* __restrict__ counts,
-                                        const int64_t* __restrict__ index, const T2* __restrict__ inv,
-                                        const T2* __restrict__ xr, T2* __restrict__ yr, int64_t t) {
-    const int S = SC ? SC : S_;
+__device__ __forceinline__ void bj_rows(const BjShape& g, const T2* __restrict__ xr, T2* __restrict__ yr, int64_t t) {
+    const int S = SC ? SC : g.S;
+    const int nblocks = g.nbx * g.nby;
     const int blk = (int)(t / S), r = (int)(t % S);
+    const bool in = t < (int64_t)nblocks * S;
+    const int J = in ? blk / g.nbx : 0, I = in ? blk - J * g.nbx : 0;
+    const int lx = I == g.nbx - 1, ly = J == g.nby - 1;
+    const BlockLayout l = block_layout(g, lx, ly);
+    const int cnt = in ? l.count() : 0;
+    const T2* inv = static_cast<const T2*>(g.inv) + (lx + 2 * ly) * S * S;
+    auto index = [&](int u) -> int64_t {
+        int dir, i, j;
+        l.unknown(u, dir, i, j);
+        i += I * g.bx;
+        j += J * g.by;
+        return dir ? g.nx_roof + i + (int64_t)g.cx * j : i + (int64_t)(g.cx - 1) * j;
+    };
+    const bool row = r < cnt;
     if ((32 % S) == 0) {
         // every lane reaches the shuffles: blocks past the end and rows past a block's count carry zeros
-        const bool in = blk < nblocks;
-        const int cnt = in ? counts[blk] : 0;
-        const int64_t* idx = index + (int64_t)blk * S;
-        const bool row = in && r < cnt;
-        const T2 mine = row ? xr[idx[r]] : czero<T2>();
-        const T2* col = inv + (int64_t)blk * S * S + r;
+        const int64_t at = row ? index(r) : 0;
+        const T2 mine = row ? xr[at] : czero<T2>();
         const int base = (int)(threadIdx.x & 31) - r;  // the block's first lane (blocks align with warps)
         T2 acc = czero<T2>();
 #pragma unroll 16
@@ -193,51 +213,42 @@ __device__ __forceinline__ void bj_rows(int nblocks, int S_, const int* __restri
             T2 v;
             v.x = __shfl_sync(0xffffffffu, mine.x, base + c);
             v.y = __shfl_sync(0xffffffffu, mine.y, base + c);
-            if (c < cnt && row) acc = cadd(acc, cmul(col[c * S], v));
+            if (c < cnt && row) acc = cadd(acc, cmul(__ldg(&inv[c * S + r]), v));
         }
-        if (row) yr[idx[r]] = acc;
+        if (row) yr[at] = acc;
         return;
     }
-    if (blk >= nblocks) return;
-    const int cnt = counts[blk];
-    if (r >= cnt) return;
-    const int64_t* idx = index + (int64_t)blk * S;
-    const T2* col = inv + (int64_t)blk * S * S + r;
+    if (!row) return;
     T2 acc = czero<T2>();
     // unrolled so that the loads of all columns are in flight together (the order of the sum is unchanged)
 #pragma unroll 8
-    for (int c = 0; c < cnt; ++c) acc = cadd(acc, cmul(col[c * S], xr[idx[c]]));
-    yr[idx[r]] = acc;
+    for (int c = 0; c < cnt; ++c) acc = cadd(acc, cmul(__ldg(&inv[c * S + r]), xr[index(c)]));
+    yr[index(r)] = acc;
 }
 
 template <typename T2>
-__global__ void k_bj_apply(int nblocks, int S, const int* __restrict__ counts, const int64_t* __restrict__ index,
-                           const T2* __restrict__ inv, const T2* __restrict__ x, T2* __restrict__ y, int64_t n,
-                           const int* skip, int stride) {
+__global__ void k_bj_apply(const BjShape g, const T2* __restrict__ x, T2* __restrict__ y, int64_t n, const int* skip,
+                           int stride) {
     const int rhs = blockIdx.y;
     if (skip && skip[(int64_t)rhs * stride]) return;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (S == 8) bj_rows<T2, 8>(nblocks, S, counts, index, inv, x + rhs * n, y + rhs * n, t);
-    else bj_rows<T2, 0>(nblocks, S, counts, index, inv, x + rhs * n, y + rhs * n, t);
+    if (g.S == 8) bj_rows<T2, 8>(g, x + rhs * n, y + rhs * n, t);
+    else bj_rows<T2, 0>(g, x + rhs * n, y + rhs * n, t);
 }
 
 // k_bj_apply for a batch of block-Jacobi operators: right-hand side k takes entry k's blocks.
 template <typename T2>
-__global__ void k_bj_apply_batch(const BjEntry* __restrict__ entries, const T2* __restrict__ x, T2* __restrict__ y,
+__global__ void k_bj_apply_batch(const BjShape* __restrict__ entries, const T2* __restrict__ x, T2* __restrict__ y,
                                  int64_t stride, const int* skip, int skip_stride) {
     const int rhs = blockIdx.y;
     if (skip && skip[(int64_t)rhs * skip_stride]) return;
-    const BjEntry e = entries[rhs];
+    const BjShape e = entries[rhs];
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e.S == 8)
-        bj_rows<T2, 8>(e.nblocks, e.S, e.counts, e.index, static_cast<const T2*>(e.inv), x + rhs * stride,
-                       y + rhs * stride, t);
-    else
-        bj_rows<T2, 0>(e.nblocks, e.S, e.counts, e.index, static_cast<const T2*>(e.inv), x + rhs * stride,
-                       y + rhs * stride, t);
+    if (e.S == 8) bj_rows<T2, 8>(e, x + rhs * stride, y + rhs * stride, t);
+    else bj_rows<T2, 0>(e, x + rhs * stride, y + rhs * stride, t);
 }
 
-int apply_block_jacobi_batch(const BjEntry* entries, int count, int max_blocks, int S, int precision, const void* x,
+int apply_block_jacobi_batch(const BjShape* entries, int count, int max_blocks, int S, int precision, const void* x,
                              void* y, int64_t stride, cudaStream_t s, SkipFlags skip) {
     const int64_t threads = (int64_t)max_blocks * S;
     const dim3 g((unsigned)((threads + 255) / 256), count);
@@ -253,35 +264,28 @@ int apply_block_jacobi_batch(const BjEntry* entries, int count, int max_blocks, 
 }
 
 struct BlockJacobi : LinearOp {
-    int nblocks = 0;
-    int S = kMaxBlockUnknowns;  // unknowns a block at most (packed stride)
-    DeviceBuffer counts, index, inv;
+    BjShape shape;
+    DeviceBuffer inv;  // [kBlockClasses][S][S]
     int apply(const void* x, void* y, int nrhs, cudaStream_t s, SkipFlags skip) override {
-        const int64_t threads = (int64_t)nblocks * S;
+        const int64_t threads = (int64_t)shape.nbx * shape.nby * shape.S;
         dim3 g((unsigned)((threads + 255) / 256), nrhs);
         if (precision == RTM_FP64)
-            k_bj_apply<double2><<<g, 256, 0, s>>>(nblocks, S, counts.as<int>(), index.as<int64_t>(), inv.as<double2>(),
-                                                  static_cast<const double2*>(x), static_cast<double2*>(y), n, skip.ptr,
-                                                  skip.stride);
+            k_bj_apply<double2><<<g, 256, 0, s>>>(shape, static_cast<const double2*>(x), static_cast<double2*>(y), n,
+                                                  skip.ptr, skip.stride);
         else
-            k_bj_apply<float2><<<g, 256, 0, s>>>(nblocks, S, counts.as<int>(), index.as<int64_t>(), inv.as<float2>(),
-                                                 static_cast<const float2*>(x), static_cast<float2*>(y), n, skip.ptr,
-                                                 skip.stride);
+            k_bj_apply<float2><<<g, 256, 0, s>>>(shape, static_cast<const float2*>(x), static_cast<float2*>(y), n,
+                                                 skip.ptr, skip.stride);
         count_launch();
         RTM_CUDA(cudaGetLastError());
         return RTM_OK;
     }
-    double stored_bytes() const override { return (double)(counts.bytes + index.bytes + inv.bytes); }
+    double stored_bytes() const override { return (double)inv.bytes; }
 };
 
-bool block_jacobi_entry(const LinearOp* op, BjEntry* out) {
+bool block_jacobi_entry(const LinearOp* op, BjShape* out) {
     const auto* bj = dynamic_cast<const BlockJacobi*>(op);
     if (!bj) return false;
-    out->nblocks = bj->nblocks;
-    out->S = bj->S;
-    out->counts = bj->counts.as<int>();
-    out->index = bj->index.as<int64_t>();
-    out->inv = bj->inv.ptr;
+    *out = bj->shape;
     return true;
 }
 
@@ -296,37 +300,31 @@ std::unique_ptr<LinearOp> make_block_jacobi(const DeviceGenerators& gen, double 
     const int64_t nx_roof = (int64_t)(cx - 1) * cy, ny_roof = (int64_t)cx * (cy - 1);
     op->n = nx_roof + ny_roof;
     op->precision = precision;
-    BjArgs g{};
+    BjShape& g = op->shape;
     g.cx = cx;
     g.cy = cy;
     g.bx = bx;
     g.by = by;
     g.nbx = (cx + bx - 1) / bx;
     g.nby = (cy + by - 1) / by;
-    g.a = size_x;
-    g.b = size_y;
-    g.E = gen.e.as<double2>();
-    g.XX = gen.xx.as<double2>();
-    g.YY = gen.yy.as<double2>();
+    g.S = 2 * bx * by;
     g.nx_roof = nx_roof;
-    op->nblocks = g.nbx * g.nby;
-    const size_t nb = (size_t)op->nblocks;
-    DeviceBuffer inv64, index16, flag;
+    DeviceBuffer flag;
     StreamSyncGuard guard(s);
-    if ((*status = op->counts.alloc(nb * sizeof(int))) != RTM_OK) return nullptr;
-    if ((*status = index16.alloc(nb * kMaxBlockUnknowns * sizeof(int64_t))) != RTM_OK) return nullptr;
-    if ((*status = inv64.alloc(nb * kMaxBlockUnknowns * kMaxBlockUnknowns * sizeof(double2))) != RTM_OK) return nullptr;
+    const size_t entries = (size_t)kBlockClasses * g.S * g.S;
+    if ((*status = op->inv.alloc(entries * (precision == RTM_FP64 ? sizeof(double2) : sizeof(float2)))) != RTM_OK)
+        return nullptr;
     if ((*status = flag.alloc(sizeof(int))) != RTM_OK) return nullptr;
     if ((*status = check_cuda(cudaMemsetAsync(flag.ptr, 0, sizeof(int), s), "block-Jacobi flag")) != RTM_OK)
         return nullptr;
-    g.counts = op->counts.as<int>();
-    g.index = index16.as<int64_t>();
-    g.inv = inv64.as<double2>();
-    g.singular = flag.as<int>();
-    // a preference only: a device that declines it runs the build all the same
-    if (cudaFuncSetAttribute(k_bj_build, cudaFuncAttributePreferredSharedMemoryCarveout, 0) != cudaSuccess)
-        (void)cudaGetLastError();
-    k_bj_build<<<(unsigned)((nb + 63) / 64), 64, 0, s>>>(g);
+    g.inv = op->inv.ptr;
+    const double2 *E = gen.e.as<double2>(), *XX = gen.xx.as<double2>(), *YY = gen.yy.as<double2>();
+    if (precision == RTM_FP64)
+        k_bj_build<double2><<<kBlockClasses, kBuildThreads, 0, s>>>(g, E, XX, YY, size_x, size_y,
+                                                                    op->inv.as<double2>(), flag.as<int>());
+    else
+        k_bj_build<float2><<<kBlockClasses, kBuildThreads, 0, s>>>(g, E, XX, YY, size_x, size_y, op->inv.as<float2>(),
+                                                                   flag.as<int>());
     count_launch();
     if ((*status = check_cuda(cudaGetLastError(), "block-Jacobi build launch")) != RTM_OK) return nullptr;
     int bad = 0;
@@ -340,25 +338,6 @@ std::unique_ptr<LinearOp> make_block_jacobi(const DeviceGenerators& gen, double 
     }
     if (bad) {
         *status = fail(RTM_ERR_SINGULAR, "a block of the block-Jacobi preconditioner is singular");
-        return nullptr;
-    }
-    const int S = 2 * bx * by;
-    op->S = S;
-    const int64_t cnt = (int64_t)nb * S * S;
-    if ((*status = op->index.alloc(nb * S * sizeof(int64_t))) != RTM_OK) return nullptr;
-    if ((*status = op->inv.alloc(cnt * (precision == RTM_FP64 ? sizeof(double2) : sizeof(float2)))) != RTM_OK)
-        return nullptr;
-    const unsigned pb = (unsigned)std::min<int64_t>((cnt + 255) / 256, 2368);
-    if (precision == RTM_FP64)
-        k_bj_pack<double2><<<pb, 256, 0, s>>>(op->nblocks, S, inv64.as<double2>(), index16.as<int64_t>(),
-                                              op->inv.as<double2>(), op->index.as<int64_t>());
-    else
-        k_bj_pack<float2><<<pb, 256, 0, s>>>(op->nblocks, S, inv64.as<double2>(), index16.as<int64_t>(),
-                                             op->inv.as<float2>(), op->index.as<int64_t>());
-    count_launch();
-    if ((e = cudaGetLastError()) == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        *status = cuda_fail(e, "block-Jacobi packing");
         return nullptr;
     }
     *status = RTM_OK;

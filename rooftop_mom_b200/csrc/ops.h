@@ -33,19 +33,19 @@ struct DeviceGenerators;
 std::unique_ptr<LinearOp> make_block_jacobi(const DeviceGenerators& g, double size_x, double size_y, int bx, int by,
                                             int precision, cudaStream_t s, int* status);
 
-// The device arrays of a block-Jacobi operator (make_block_jacobi), for batched applies: blocks, their
-// packed size S, unknowns per block, rooftop indices [nblocks][S] and inverses [nblocks][S][S] (column-major).
-struct BjEntry {
-    int nblocks = 0, S = 0;
-    const int* counts = nullptr;
-    const int64_t* index = nullptr;
+// A block-Jacobi operator as its apply needs it: faces, blocks of bx x by faces in nbx columns and nby rows, the
+// packed size S = 2 bx by, the x-directed rooftops, and the inverses of the four block classes
+// ([class][S][S], column-major; class (last column) + 2 (last row)) in the operator's precision.
+struct BjShape {
+    int cx = 0, cy = 0, bx = 1, by = 1, nbx = 0, nby = 0, S = 0;
+    int64_t nx_roof = 0;
     const void* inv = nullptr;
 };
 // False when op is not a block-Jacobi operator.
-bool block_jacobi_entry(const LinearOp* op, BjEntry* out);
+bool block_jacobi_entry(const LinearOp* op, BjShape* out);
 // y = M_k x for count block-Jacobi operators at once (one launch; entry k's vectors start at k * stride),
 // entries a device table; max_blocks the most blocks of an entry.
-int apply_block_jacobi_batch(const BjEntry* entries, int count, int max_blocks, int S, int precision, const void* x,
+int apply_block_jacobi_batch(const BjShape* entries, int count, int max_blocks, int S, int precision, const void* x,
                              void* y, int64_t stride, cudaStream_t s, SkipFlags skip);
 
 // Precision conversion of complex vectors on the device.
