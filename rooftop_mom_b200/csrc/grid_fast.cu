@@ -190,6 +190,12 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_y_fwd(const Gri
         for (int k2 = 0; k2 < R2; ++k2) dst[(int64_t)((t + R2 * s) + R1 * k2) * a.P] = v[s * R2 + k2];
 }
 
+// The spectra of a generator are even in both frequencies (its embedding is even): of the subband with parity p
+// on n frequencies, f = 2 m + p, entry m equals entry n - m - p (mod n). The x-mix reads the lower of the two,
+// so of the 12 P Q stored values a product touches 3 P Q, which stay in L2 between products (FP32 1024 x 1024:
+// 25 MB instead of 100).
+__device__ __forceinline__ int even_freq(int m, int p, int n) { return min(m, n - m - p); }
+
 // x-mix, direct form (one CTA per TEAMS y frequencies; inputs loaded straight into registers, the spectra
 // read in the mix): teams of four groups (component c, x subband px) per y frequency j of subband py. Thread
 // index t + R2 (team * 4 + 2 px + c). Forward transform along x of W mod_x^px, the 2x2 block mix
@@ -235,7 +241,7 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
     __syncthreads();
     if (on) {
         const int sub = px + 2 * py;
-        const T2* spec = pd.spec + (int64_t)(sub * 3) * QP + (int64_t)j * NP;
+        const T2* spec = pd.spec + (int64_t)(sub * 3) * QP + (int64_t)even_freq(j, py, Q) * NP;
         const T2* ux = px ? a.ux1 : a.ux0;
         const T2 vv = __ldg(&(py ? a.vy1 : a.vy0)[j]);
         const T cv = (vv.x * vv.x + vv.y * vv.y) * pd.inv_b2;
@@ -244,8 +250,9 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
 #pragma unroll
             for (int k2 = 0; k2 < R2; ++k2) {
                 const int k = (t + R2 * s) + R1 * k2;
-                const T2 E = __ldg(&spec[k]);
-                const T2 M = __ldg(&spec[(1 + c) * QP + k]);
+                const int ke = even_freq(k, px, NP);
+                const T2 E = __ldg(&spec[ke]);
+                const T2 M = __ldg(&spec[(1 + c) * QP + ke]);
                 const T2 uu = __ldg(&ux[k]);
                 const T cu = (uu.x * uu.x + uu.y * uu.y) * pd.inv_a2;
                 // qc = -u conj(v) / (ab): XY = qc E, YX = conj(qc) E
@@ -294,10 +301,12 @@ template <typename T, int NP> struct MixShape {
     static constexpr int R1 = Shape<NP>::R1, R2 = Shape<NP>::R2;
     static constexpr int TEAMS = Fast<T>::threads / (4 * R2), LB = R1 * (R2 + 1);
     using T2 = typename Cx<T>::T2;
-    // line buffers [4 TEAMS][LB], W rows [2 c][TEAMS][NP], spectra rows [2 px][3 kind][TEAMS][NP]
+    // line buffers [4 TEAMS][LB], W rows [2 c][TEAMS][NP], spectra rows [2 px][3 kind][TEAMS][NS], the lower half
+    // of each row (even_freq), padded to 16 bytes
+    static constexpr int NS = NP / 2 + 2;
     static constexpr size_t lines = (size_t)4 * TEAMS * LB * sizeof(T2);
     static constexpr size_t wrows = (size_t)2 * TEAMS * NP * sizeof(T2);
-    static constexpr size_t srows = (size_t)6 * TEAMS * NP * sizeof(T2);
+    static constexpr size_t srows = (size_t)6 * TEAMS * NS * sizeof(T2);
     static constexpr size_t smem = lines + wrows + srows;
     static constexpr int blocks = 2 * smem <= 220 * 1024 ? 2 : 1;  // CTAs per SM the registers are sized for
 };
@@ -306,9 +315,11 @@ template <typename T, int NP>
 __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k_fast_x_mix_pipe(const GridArgs<T> a, int iters) {
     using M = MixShape<T, NP>;
     using T2 = typename Cx<T>::T2;
-    constexpr int R1 = M::R1, R2 = M::R2, S = R1 / R2, TEAMS = M::TEAMS, LB = M::LB;
+    constexpr int R1 = M::R1, R2 = M::R2, S = R1 / R2, TEAMS = M::TEAMS, LB = M::LB, NS = M::NS;
     constexpr unsigned BLOCK = TEAMS * NP * sizeof(T2);  // TEAMS consecutive rows of one grid
-    static_assert(BLOCK % 16 == 0 && M::lines % 16 == 0 && M::wrows % 16 == 0, "bulk copies need 16-byte units");
+    constexpr unsigned HALF = NS * sizeof(T2);           // the lower half of a spectra row
+    static_assert(BLOCK % 16 == 0 && HALF % 16 == 0 && M::lines % 16 == 0 && M::wrows % 16 == 0,
+                  "bulk copies need 16-byte units");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T2* sm = reinterpret_cast<T2*>(smem_raw);
     T2* wst = reinterpret_cast<T2*>(smem_raw + M::lines);
@@ -339,12 +350,15 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
         }
         if (spectra) {
             ++issued[1];
-            mbar_expect_tx(&bar[1], 6 * BLOCK);
+            mbar_expect_tx(&bar[1], 6 * TEAMS * HALF);
             const T2* sp = a.plates ? a.plates[rhs].spec : a.spec;
             for (int q = 0; q < 2; ++q)
                 for (int kind = 0; kind < 3; ++kind)
-                    bulk_load(sst + (q * 3 + kind) * TEAMS * NP,
-                              sp + (int64_t)((q + 2 * py) * 3 + kind) * QP + (int64_t)j0 * NP, BLOCK, &bar[1]);
+                    for (int e = 0; e < TEAMS; ++e)
+                        bulk_load(sst + ((q * 3 + kind) * TEAMS + e) * NS,
+                                  sp + (int64_t)((q + 2 * py) * 3 + kind) * QP +
+                                      (int64_t)even_freq(j0 + e, py, Q) * NP,
+                                  HALF, &bar[1]);
         }
     };
     if (tid == 0) {
@@ -387,8 +401,8 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
         if (__syncthreads_or(!mbar_wait(&bar[1], done[1] & 1, a.fault))) break;
         ++done[1];
         {
-            const T2* Es = sst + (px * 3 * TEAMS + team) * NP;
-            const T2* Ms = sst + ((px * 3 + 1 + c) * TEAMS + team) * NP;
+            const T2* Es = sst + (px * 3 * TEAMS + team) * NS;
+            const T2* Ms = sst + ((px * 3 + 1 + c) * TEAMS + team) * NS;
             const T2 vv = __ldg(&(py ? a.vy1 : a.vy0)[j]);
             const T cv = (vv.x * vv.x + vv.y * vv.y) * pd.inv_b2;
 #pragma unroll
@@ -396,8 +410,9 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
 #pragma unroll
                 for (int k2 = 0; k2 < R2; ++k2) {
                     const int k = (t + R2 * s) + R1 * k2;
-                    const T2 E = Es[k];
-                    const T2 Mk = Ms[k];
+                    const int ke = even_freq(k, px, NP);
+                    const T2 E = Es[ke];
+                    const T2 Mk = Ms[ke];
                     const T2 uu = __ldg(&ux[k]);
                     const T cu = (uu.x * uu.x + uu.y * uu.y) * pd.inv_a2;
                     // qc = -u conj(v) / (ab): XY = qc E, YX = conj(qc) E
