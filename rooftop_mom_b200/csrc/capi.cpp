@@ -46,19 +46,13 @@ int check_plane_wave(const double* d, const double* p) {
 
 namespace {
 
-int make_stream(cudaStream_t* s) {
-    RTM_CUDA(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
-    return RTM_OK;
-}
+int make_stream(cudaStream_t* s) { return stream_acquire(s); }
 
-// A stream made for one call; declared before the call's staging buffers, it outlives them.
+// A stream of one call; declared before the call's staging buffers, it outlives them.
 struct CallStream {
     cudaStream_t s = nullptr;
     ~CallStream() {
-        if (s) {
-            cudaStreamSynchronize(s);
-            cudaStreamDestroy(s);
-        }
+        if (s) stream_release(s);
     }
 };
 
@@ -693,7 +687,7 @@ struct rtm_plate_batch {
         if (stream) cudaStreamSynchronize(stream);
         op.reset();
         pc.reset();
-        if (stream) cudaStreamDestroy(stream);
+        if (stream) stream_release(stream);
     }
 };
 

@@ -16,7 +16,7 @@ struct rtm_generators {
         g.xx.reset();
         g.yy.reset();
         g.e.reset();
-        if (stream) cudaStreamDestroy(stream);
+        if (stream) rtm::stream_release(stream);
     }
 };
 
@@ -29,7 +29,7 @@ struct rtm_operator {
     ~rtm_operator() {
         if (stream) cudaStreamSynchronize(stream);
         op.reset();
-        if (stream) cudaStreamDestroy(stream);
+        if (stream) rtm::stream_release(stream);
     }
 };
 
@@ -40,7 +40,7 @@ struct rtm_preconditioner {
     ~rtm_preconditioner() {
         if (stream) cudaStreamSynchronize(stream);
         op.reset();
-        if (stream) cudaStreamDestroy(stream);
+        if (stream) rtm::stream_release(stream);
     }
 };
 

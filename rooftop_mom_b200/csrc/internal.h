@@ -92,6 +92,14 @@ struct StreamSyncGuard {
     ~StreamSyncGuard() { cudaStreamSynchronize(s); }
 };
 
+// Non-blocking streams from a pool of idle ones, since making and destroying one costs about 114 us on the host
+// and every handle has its own. stream_release synchronises the stream, then keeps it for the next handle on its
+// device (at most kIdleStreams a device) or destroys it. Safe from several threads; a stream has one owner at a
+// time.
+constexpr int kIdleStreams = 32;
+int stream_acquire(cudaStream_t* s);
+void stream_release(cudaStream_t s);
+
 // ---------------------------------------------------------------------------------------------
 // FFT plans: a length n factorised into radices; twiddle tables exp(-2 pi i m / n), m < n, in
 // FP64 and FP32, computed on the host in long double and kept on the device for the life of the
@@ -137,7 +145,6 @@ template <> struct Cx<float> { using T2 = float2; };
 
 // Host FP64 helpers used by the assembler set-up.
 void gauss_legendre(int order, double a, double b, std::vector<double>& points, std::vector<double>& weights);
-void power_moments(double size_x, double size_y, int power, double out[7][4]);
 void extracted_moments(double size_x, double size_y, double k, double out[7][4]);
 
 int fast_fft_size(int count);

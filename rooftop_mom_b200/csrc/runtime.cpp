@@ -149,6 +149,46 @@ void DeviceBuffer::reset() {
 }
 
 // ---------------------------------------------------------------------------------------------
+// Idle streams by device, and the device of every stream handed out.
+static std::mutex g_streams_mu;
+static std::vector<cudaStream_t> g_idle_streams[64];
+static std::map<cudaStream_t, int> g_stream_device;
+
+int stream_acquire(cudaStream_t* s) {
+    *s = nullptr;
+    int dev = 0;
+    RTM_CUDA(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> lk(g_streams_mu);
+        auto& idle = g_idle_streams[dev & 63];
+        if (dev < 64 && !idle.empty()) {
+            *s = idle.back();
+            idle.pop_back();
+            return RTM_OK;
+        }
+    }
+    RTM_CUDA(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+    std::lock_guard<std::mutex> lk(g_streams_mu);
+    g_stream_device[*s] = dev;
+    return RTM_OK;
+}
+
+void stream_release(cudaStream_t s) {
+    const bool sound = cudaStreamSynchronize(s) == cudaSuccess;
+    {
+        std::lock_guard<std::mutex> lk(g_streams_mu);
+        auto it = g_stream_device.find(s);
+        const int dev = it == g_stream_device.end() ? 64 : it->second;
+        if (sound && dev < 64 && (int)g_idle_streams[dev].size() < kIdleStreams) {
+            g_idle_streams[dev].push_back(s);
+            return;
+        }
+        if (it != g_stream_device.end()) g_stream_device.erase(it);
+    }
+    cudaStreamDestroy(s);
+}
+
+// ---------------------------------------------------------------------------------------------
 // FFT plans and tables.
 int fast_fft_size(int count) {
     // generateFastFFTSize.m:11-15: the smallest size >= count with prime factors <= 7.
@@ -363,7 +403,7 @@ int shift_factors(int n, int parity, const double2** out64, const float2** out32
 // ---------------------------------------------------------------------------------------------
 // Gauss-Legendre points and weights on [a, b] by Newton's method on P_n (same rule as the
 // Golub-Welsch eigenvalue method of generateGaussLegendre1D.m:16-25, to rounding).
-void gauss_legendre(int order, double a, double b, std::vector<double>& points, std::vector<double>& weights) {
+static void gauss_legendre_unit(int order, std::vector<double>& points, std::vector<double>& weights) {
     points.assign(order, 0.0);
     weights.assign(order, 0.0);
     const long double pi = 3.141592653589793238462643383279502884L;
@@ -403,6 +443,26 @@ void gauss_legendre(int order, double a, double b, std::vector<double>& points, 
             points[order / 2] = 0.0;
             weights[order / 2] = (double)(2 / (dp * dp));
         }
+    }
+}
+
+// The rules of an order on [a, b]. The unit rules of orders up to kCachedOrder are computed once a process (an
+// assembly asks for seven, about 1 ms of long-double Newton steps otherwise).
+void gauss_legendre(int order, double a, double b, std::vector<double>& points, std::vector<double>& weights) {
+    constexpr int kCachedOrder = 64;
+    static std::mutex mu;
+    static std::map<int, std::pair<std::vector<double>, std::vector<double>>> unit;
+    if (order > kCachedOrder) {
+        gauss_legendre_unit(order, points, weights);
+    } else {
+        std::lock_guard<std::mutex> lk(mu);
+        auto it = unit.find(order);
+        if (it == unit.end()) {
+            gauss_legendre_unit(order, points, weights);
+            it = unit.emplace(order, std::make_pair(points, weights)).first;
+        }
+        points = it->second.first;
+        weights = it->second.second;
     }
     for (int i = 0; i < order; ++i) {
         points[i] = (a + b) / 2 + (b - a) / 2 * points[i];
@@ -459,35 +519,47 @@ static double monomial(int power, int m, int n, double a, double b) {
     return NAN;
 }
 
-// rect[m][n][iu][iv]: integral of u^m v^n R^power over [iu, iu+1] x ratio [iv, iv+1].
-static void rectangles(int power, double ratio, double rect[4][2][2][2]) {
-    for (int m = 0; m < 4; ++m)
-        for (int n = 0; n < 2; ++n) {
-            double c[3][3];
-            for (int k = 0; k < 3; ++k)
-                for (int l = 0; l < 3; ++l) c[k][l] = monomial(power, m, n, (double)k, ratio * l);
-            for (int k = 0; k < 2; ++k)
-                for (int l = 0; l < 2; ++l) rect[m][n][k][l] = (c[k + 1][l + 1] - c[k][l + 1]) - (c[k + 1][l] - c[k][l]);
-        }
+// rect[q][m][n][iu][iv]: integral of u^m v^n R^power over [iu, iu+1] x ratio [iv, iv+1], power = kPowers[q]. The
+// rectangles away from the corner take a 20 x 20-point rule, all powers and monomials at once from one square root
+// a point (a pow per factor had cost 1.2 ms an assembly).
+static const int kPowers[3] = {-1, 1, 3};
+static void rectangles(double ratio, double rect[3][4][2][2][2]) {
+    for (int q = 0; q < 3; ++q)
+        for (int m = 0; m < 4; ++m)
+            for (int n = 0; n < 2; ++n) {
+                double c[3][3];
+                for (int k = 0; k < 3; ++k)
+                    for (int l = 0; l < 3; ++l) c[k][l] = monomial(kPowers[q], m, n, (double)k, ratio * l);
+                for (int k = 0; k < 2; ++k)
+                    for (int l = 0; l < 2; ++l)
+                        rect[q][m][n][k][l] = (c[k + 1][l + 1] - c[k][l + 1]) - (c[k + 1][l] - c[k][l]);
+            }
     std::vector<double> pts, w;
     gauss_legendre(20, 0.0, 1.0, pts, w);
     for (int k = 0; k < 2; ++k)
         for (int l = 0; l < 2; ++l) {
             if (std::hypot((double)k, ratio * l) < std::max(1.0, ratio)) continue;
-            for (int m = 0; m < 4; ++m)
-                for (int n = 0; n < 2; ++n) {
-                    double s = 0;
-                    for (int i = 0; i < 20; ++i) {
-                        double inner = 0;
-                        const double u = k + pts[i];
-                        for (int j = 0; j < 20; ++j) {
-                            const double v = ratio * (l + pts[j]);
-                            inner += w[j] * std::pow(u, m) * std::pow(v, n) * std::pow(std::sqrt(u * u + v * v), power);
-                        }
-                        s += w[i] * inner;
+            double s[3][4][2] = {};
+            for (int i = 0; i < 20; ++i) {
+                double inner[3][2] = {};
+                const double u = k + pts[i];
+                for (int j = 0; j < 20; ++j) {
+                    const double v = ratio * (l + pts[j]);
+                    const double r2 = u * u + v * v, r = std::sqrt(r2);
+                    const double f[3] = {1.0 / r, r, r * r2};
+                    for (int q = 0; q < 3; ++q) {
+                        inner[q][0] += w[j] * f[q];
+                        inner[q][1] += w[j] * v * f[q];
                     }
-                    rect[m][n][k][l] = ratio * s;
                 }
+                double um = 1;
+                for (int m = 0; m < 4; ++m, um *= u)
+                    for (int q = 0; q < 3; ++q)
+                        for (int n = 0; n < 2; ++n) s[q][m][n] += w[i] * (um * inner[q][n]);
+            }
+            for (int q = 0; q < 3; ++q)
+                for (int m = 0; m < 4; ++m)
+                    for (int n = 0; n < 2; ++n) rect[q][m][n][k][l] = ratio * s[q][m][n];
         }
 }
 
@@ -522,10 +594,8 @@ static void compose_part(const double* weight, int len, int part, int offset, do
     }
 }
 
-static void along_x(double a, double b, int power, double out[4][4]) {
+static void along_x(double a, double b, int power, const double rect[4][2][2][2], double out[4][4]) {
     const double ratio = b / a;
-    double rect[4][2][2][2];
-    rectangles(power, ratio, rect);
     for (int k = 0; k < 4; ++k)
         for (int l = 0; l < 4; ++l) {
             double acc = 0;
@@ -545,10 +615,12 @@ static void along_x(double a, double b, int power, double out[4][4]) {
         }
 }
 
-void power_moments(double size_x, double size_y, int power, double out[7][4]) {
+// rx, ry: the rectangles of kPowers' entry `power` for the ratios size_y / size_x and size_x / size_y.
+static void power_moments(double size_x, double size_y, int power, const double rx[4][2][2][2],
+                          const double ry[4][2][2][2], double out[7][4]) {
     double ax[4][4], ay[4][4];
-    along_x(size_x, size_y, power, ax);
-    along_x(size_y, size_x, power, ay);
+    along_x(size_x, size_y, power, rx, ax);
+    along_x(size_y, size_x, power, ry, ay);
     static const int perm[4] = {0, 2, 1, 3};
     for (int l = 0; l < 4; ++l) {
         for (int k = 0; k < 4; ++k) out[k][l] = ax[k][l];
@@ -557,10 +629,11 @@ void power_moments(double size_x, double size_y, int power, double out[7][4]) {
 }
 
 void extracted_moments(double size_x, double size_y, double k, double out[7][4]) {
-    double m1[7][4], p1[7][4], p3[7][4];
-    power_moments(size_x, size_y, -1, m1);
-    power_moments(size_x, size_y, 1, p1);
-    power_moments(size_x, size_y, 3, p3);
+    double m[3][7][4], rx[3][4][2][2][2], ry[3][4][2][2][2];
+    rectangles(size_y / size_x, rx);
+    rectangles(size_x / size_y, ry);
+    for (int q = 0; q < 3; ++q) power_moments(size_x, size_y, kPowers[q], rx[q], ry[q], m[q]);
+    const auto &m1 = m[0], &p1 = m[1], &p3 = m[2];
     for (int r = 0; r < 7; ++r)
         for (int c = 0; c < 4; ++c) out[r][c] = m1[r][c] - k * k / 2 * p1[r][c] + k * k * k * k / 24 * p3[r][c];
 }
