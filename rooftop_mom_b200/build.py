@@ -15,6 +15,8 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "librtm.so")
 OBJ = os.path.join(HERE, "_build")
 SOURCES = ["runtime.cpp", "capi.cpp", "server.cpp", "grid.cu", "grid_fast.cu", "assembly.cu", "krylov.cu", "ops.cu", "excitation.cu", "fixed_scratch.cu", "fault.cu", "tune.cpp", "batch.cu"]
+# sources compiled once for each form, so that their kernels compile side by side: object name -> (source, defines)
+FORMS = {f"grid_reg.{k}": ("grid_reg.cu", [f"-DRTM_REG_FORM={k}"]) for k in range(8)}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
          "-Wno-deprecated-gpu-targets"]
@@ -40,12 +42,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(HERE, "..", "include", "rtm.h"))
     jobs = []
-    for src in SOURCES:
+    units = {**FORMS, **{src: (src, []) for src in SOURCES}}
+    for name, (src, defines) in units.items():
         path = os.path.join(CSRC, src)
-        obj = os.path.join(OBJ, src + ".o")
+        obj = os.path.join(OBJ, name + ".o")
         if force or _stale(obj, [path] + headers):
-            cmd = [nvcc, *FLAGS, *ARCH, "-c", path, "-o", obj]
-            jobs.append((src, cmd))
+            cmd = [nvcc, *FLAGS, *ARCH, *defines, "-c", path, "-o", obj]
+            jobs.append((name, cmd))
 
     def run(job):
         src, cmd = job
@@ -58,7 +61,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
     with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as ex:
         list(ex.map(run, jobs))
-    objs = [os.path.join(OBJ, s + ".o") for s in SOURCES]
+    objs = [os.path.join(OBJ, s + ".o") for s in units]
     if force or jobs or not os.path.exists(OUT) or _stale(OUT, objs):
         cmd = [nvcc, *ARCH, "-shared", "-o", OUT + ".tmp", *objs, "-lcudart", "-Xcompiler", "-fPIC"]
         p = subprocess.run(cmd, capture_output=True, text=True)

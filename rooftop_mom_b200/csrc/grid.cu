@@ -357,6 +357,20 @@ template <typename T> static GridArgs<T> product_args(const GridApplicator& g, S
 }
 
 template <typename T>
+static int reg_pass(int pass, const GridArgs<T>& a, const RegPlan& r, int nrhs, const void* x, void* y, cudaStream_t s) {
+    const bool wide = r.n1 > 16;
+    if (r.m != r.n)  // FP32 lines transform in FP64 there
+        return wide ? launch_reg_pass<T, double, 1, true>(pass, a, r, nrhs, x, y, s)
+                    : launch_reg_pass<T, double, 0, true>(pass, a, r, nrhs, x, y, s);
+    return wide ? launch_reg_pass<T, T, 1, false>(pass, a, r, nrhs, x, y, s)
+                : launch_reg_pass<T, T, 0, false>(pass, a, r, nrhs, x, y, s);
+}
+
+// True when both lengths of a product have a split for the register-resident kernels (grid_reg.cu). The 2 nsx
+// lines of n1 <= 36 threads an x-mix needs at least fit the CTA of every form (128 threads for n1 <= 16, 192 above).
+static bool reg_eligible(const GridApplicator& g) { return g.tP->reg.n1 > 0 && g.tQ->reg.n1 > 0; }
+
+template <typename T>
 static int apply_t(const GridApplicator& g, const void* xv, void* yv, int nrhs, cudaStream_t s, SkipFlags skip,
                    void* work, int* fault) {
     using T2 = typename Cx<T>::T2;
@@ -390,6 +404,18 @@ static int apply_t(const GridApplicator& g, const void* xv, void* yv, int nrhs, 
     }
     const int passes = g.lean ? g.nsy : 1;
     const int npy = g.lean ? 1 : g.nsy;
+    if (reg_eligible(g)) {
+        a.npy = npy;
+        for (int pass = 0; pass < passes; ++pass) {
+            a.py0 = pass;
+            a.accumulate = pass > 0;
+            RTM_TRY(reg_pass<T>(kRegYFwd, a, g.tQ->reg, nrhs, x, y, s));
+            RTM_TRY(reg_pass<T>(kRegXMix, a, g.tP->reg, nrhs, x, y, s));
+            RTM_TRY(reg_pass<T>(kRegYInv, a, g.tQ->reg, nrhs, x, y, s));
+        }
+        RTM_CUDA(cudaGetLastError());
+        return RTM_OK;
+    }
     // y passes: TI x columns per CTA (rows of 64 bytes) for every y subband at once; fewer columns
     // while the tile (plus the roots) would not fit or would need more than kMaxThreads threads.
     int ti = sizeof(T) == 8 ? 4 : 8;

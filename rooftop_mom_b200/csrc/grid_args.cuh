@@ -74,4 +74,10 @@ template <typename A> __device__ __forceinline__ bool skipped(const A& a, int rh
 template <typename T>
 int launch_fast_split(const GridArgs<T>& a, int nrhs, const void* x, void* y, const FastSchedule& f, cudaStream_t s);
 
+// One pass of a product on lines with a register-resident split (grid_reg.cu): T the stored precision, C the
+// transforms', CLS the plan's codelet class (n1 <= 16: 0), BLUE a Bluestein convolution.
+enum RegPass { kRegYFwd = 0, kRegXMix = 1, kRegYInv = 2 };
+template <typename T, typename C, int CLS, bool BLUE>
+int launch_reg_pass(int pass, GridArgs<T> a, const RegPlan& r, int nrhs, const void* x, void* y, cudaStream_t s);
+
 }  // namespace rtm

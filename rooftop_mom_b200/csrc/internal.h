@@ -124,8 +124,23 @@ struct FftPlan {
     const float2* twm32;
 };
 
+// A length's split for the register-resident transforms (regfft.cuh): m = n1 n2 with n1 >= n2, both codelet
+// lengths; m == n, or m >= 2 n - 1 for a Bluestein convolution (chirp and kernel spectrum then set). n1 == 0: the
+// length has none.
+constexpr int kRegMax = 1024;
+struct RegPlan {
+    int n, m, n1, n2;
+    const double2* tw64;  // exp(-2 pi i k / m), k < m
+    const float2* tw32;
+    const double2* chirp64;  // exp(-i pi (j^2 mod 2n) / n), j < n
+    const float2* chirp32;
+    const double2* kern64;  // DFT_m of exp(+i pi d^2 / n) wrapped to length m, divided by m
+    const float2* kern32;
+};
+
 struct FftTables {
     FftPlan plan;
+    RegPlan reg;
     const double2* tw64;   // n entries
     const float2* tw32;
     const double2* mod64;  // exp(-i pi d / n), d < n (the odd-subband modulation)

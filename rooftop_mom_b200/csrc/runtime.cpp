@@ -224,6 +224,79 @@ static bool make_plan(int n, FftPlan& p) {
     return true;
 }
 
+// The codelet lengths of the register-resident transforms by class (regfft.cuh): n1 of class 0 and 1, n2 <= n1.
+static const std::vector<int> kRegN1[2] = {{4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16},
+                                           {18, 20, 21, 24, 25, 27, 28, 30, 32, 35, 36}};
+static const std::vector<int> kRegN2[2] = {{3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16},
+                                           {5, 7, 9, 10, 14, 15, 16, 18, 20, 21, 24, 25, 27, 28, 30, 32}};
+
+// The split of m with the smallest n1 (the fewest values a thread holds); false when m has none.
+static bool reg_split(int m, int* n1, int* n2) {
+    for (int c = 0; c < 2; ++c)
+        for (int a : kRegN1[c]) {
+            if (m % a) continue;
+            const int b = m / a;
+            if (b <= a && std::find(kRegN2[c].begin(), kRegN2[c].end(), b) != kRegN2[c].end()) {
+                *n1 = a;
+                *n2 = b;
+                return true;
+            }
+        }
+    return false;
+}
+
+// DFT of a length m = n1 n2 in long double (host; the kernel spectrum of a Bluestein split), four-step.
+static void host_dft_split(std::vector<std::complex<long double>>& x, int n1, int n2) {
+    const int m = n1 * n2;
+    const long double pi = 3.141592653589793238462643383279502884L;
+    std::vector<std::complex<long double>> w(m), y(m), out(m);
+    for (int k = 0; k < m; ++k) {
+        const long double a = -2.0L * pi * (long double)k / (long double)m;
+        w[k] = {cosl(a), sinl(a)};
+    }
+    for (int t = 0; t < n2; ++t)
+        for (int k1 = 0; k1 < n1; ++k1) {
+            std::complex<long double> s = 0;
+            for (int m1 = 0; m1 < n1; ++m1) s += x[n2 * m1 + t] * w[(size_t)m1 * k1 % n1 * n2];
+            y[k1 * n2 + t] = s * w[(size_t)t * k1];
+        }
+    for (int k1 = 0; k1 < n1; ++k1)
+        for (int k2 = 0; k2 < n2; ++k2) {
+            std::complex<long double> s = 0;
+            for (int t = 0; t < n2; ++t) s += y[k1 * n2 + t] * w[(size_t)t * k2 % n2 * n1];
+            out[k1 + n1 * k2] = s;
+        }
+    x.swap(out);
+}
+
+// The plan of length n for the register-resident transforms and the host values of its Bluestein tables.
+static void make_reg_plan(int n, RegPlan& p, std::vector<double2>& chirp, std::vector<double2>& kern) {
+    p = RegPlan{};
+    p.n = p.m = n;
+    if (n > kRegMax || reg_split(n, &p.n1, &p.n2)) return;
+    int m = 2 * n - 1;
+    while (m <= kRegMax && !reg_split(m, &p.n1, &p.n2)) ++m;
+    // lengths whose factors are all codelets run in the Stockham engine when they have no split
+    if (m > kRegMax || fast_fft_size(n) == n || n < 16) {
+        p.n1 = p.n2 = 0;
+        return;
+    }
+    p.m = m;
+    const long double pi = 3.141592653589793238462643383279502884L;
+    chirp.resize(n);
+    std::vector<std::complex<long double>> b(m, 0.0L);
+    for (int j = 0; j < n; ++j) {
+        const long double a = pi * (long double)((int64_t)j * j % (2 * (int64_t)n)) / (long double)n;
+        const std::complex<long double> bj(cosl(a), sinl(a));
+        chirp[j] = make_double2((double)bj.real(), (double)(-bj.imag()));
+        b[j] = bj;
+        if (j) b[m - j] = bj;
+    }
+    host_dft_split(b, p.n1, p.n2);
+    kern.resize(m);
+    for (int k = 0; k < m; ++k) kern[k] = make_double2((double)(b[k].real() / m), (double)(b[k].imag() / m));
+}
+
 struct TableKey {
     int device;
     int n;
@@ -360,6 +433,34 @@ int fft_tables(int n, const FftTables** out) {
         e.t.plan.chirp32 = d32;
         e.t.plan.kern32 = d32 + chirp.size();
         e.t.plan.twm32 = d32 + chirp.size() + kern.size();
+    }
+    RegPlan& rp = e.t.reg;
+    std::vector<double2> rchirp, rkern;
+    make_reg_plan(n, rp, rchirp, rkern);
+    if (rp.n1 && rp.m == n) {
+        rp.tw64 = e.t.tw64;
+        rp.tw32 = e.t.tw32;
+    } else if (rp.n1) {
+        // FP64 then FP32: roots of length m (m), chirp (n), kernel spectrum (m)
+        std::vector<double2> all;
+        root_table(rp.m, 2.0L, all);
+        all.insert(all.end(), rchirp.begin(), rchirp.end());
+        all.insert(all.end(), rkern.begin(), rkern.end());
+        const size_t cnt = all.size();
+        std::vector<float2> all32(cnt);
+        for (size_t i = 0; i < cnt; ++i) all32[i] = make_float2((float)all[i].x, (float)all[i].y);
+        void* mem = nullptr;
+        RTM_CUDA(cudaMalloc(&mem, cnt * (sizeof(double2) + sizeof(float2))));
+        double2* d64 = (double2*)mem;
+        float2* d32 = (float2*)(d64 + cnt);
+        RTM_CUDA(cudaMemcpy(d64, all.data(), cnt * sizeof(double2), cudaMemcpyHostToDevice));
+        RTM_CUDA(cudaMemcpy(d32, all32.data(), cnt * sizeof(float2), cudaMemcpyHostToDevice));
+        rp.tw64 = d64;
+        rp.chirp64 = d64 + rp.m;
+        rp.kern64 = rp.chirp64 + n;
+        rp.tw32 = d32;
+        rp.chirp32 = d32 + rp.m;
+        rp.kern32 = rp.chirp32 + n;
     }
     auto res = g_tables.emplace(TableKey{dev, n}, e);
     *out = &res.first->second.t;

@@ -43,3 +43,49 @@ def test_block_jacobi_of_every_block_class(shape, precision):
     for k in range(2):
         part = slice(k * rt.count, (k + 1) * rt.count)
         assert rel(got[part], want.apply(v[part])) < (1e-13 if precision == "double" else 5e-6)
+
+
+# transform lengths whose splits n1 x n2 take every codelet at least once, and the smallest and largest lengths
+SPLIT_GRIDS = [(16, 18), (20, 21), (24, 25), (27, 28), (30, 35), (36, 45), (49, 54), (60, 63), (75, 81), (98, 105),
+               (120, 125), (126, 147), (162, 175), (196, 216), (225, 243), (250, 17), (17, 270), (288, 19), (20, 315),
+               (350, 16), (16, 378), (405, 16), (18, 441), (450, 16), (16, 486), (490, 16), (16, 567), (600, 17),
+               (17, 640), (700, 16), (16, 756), (840, 16), (16, 875), (945, 16), (972, 16), (16, 1008), (343, 16)]
+
+
+@pytest.mark.parametrize("grid", SPLIT_GRIDS)
+@pytest.mark.parametrize("precision,product", [("double", "splitFFT"), ("single", "splitFFT"),
+                                               ("double", "leanSplitFFT")])
+def test_split_products_of_every_codelet(grid, precision, product):
+    """Face counts one below a transform length (a last column and row of padding) and the length itself."""
+    from oracle import spectra as S
+
+    for cx, cy in (grid, (grid[0] - 1, grid[1])):
+        R, prob, rt, gen = _setup(cx, cy)
+        v = random_vector(rt.count, seed=5)
+        want = S.split_apply(rt, S.subband_spectra(gen, rt.size_x, rt.size_y), rt.content, v)
+        got = R.Operator(prob, product=product, precision=precision).apply(v)
+        assert rel(got, want) < (1e-13 if precision == "double" else 2e-5)
+
+
+@pytest.mark.parametrize("grid", [(9, 10), (16, 17), (19, 22), (23, 18), (26, 31), (33, 37), (34, 20), (67, 61), (127, 18),
+                                  (131, 16), (18, 257), (503, 17), (17, 512), (511, 19), (514, 18), (64, 48)])
+@pytest.mark.parametrize("precision", ["double", "single"])
+def test_circulants_of_any_face_count(grid, precision):
+    """Splits, Bluestein convolutions up to their longest (512) and lengths beyond the register-resident form, for
+    one vector and for three; the embedding product (periods 2 n - 2) on the smaller grids."""
+    from oracle import preconditioner as Q, spectra as S
+
+    R, prob, rt, gen = _setup(*grid)
+    v = random_vector(3 * rt.count, seed=6)
+    spec = Q.circulant(gen, rt.size_x, rt.size_y, kernel="rChan")
+    pc = R.Preconditioner(prob, kernel="rChan", precision=precision)
+    got, one = pc.apply(v, nrhs=3), pc.apply(v[:rt.count])
+    for k in range(3):
+        part = slice(k * rt.count, (k + 1) * rt.count)
+        assert rel(got[part], S.fft_apply(rt, spec, rt.content, v[part])) < (1e-11 if precision == "double" else 2e-5)
+    assert rel(one, got[:rt.count]) < 1e-15
+    if max(grid) <= 67:
+        emb = S.embedding_spectra(gen, rt.size_x, rt.size_y)
+        want = S.fft_apply(rt, emb, rt.content, v[:rt.count])
+        got = R.Operator(prob, product="fft", precision=precision).apply(v[:rt.count])
+        assert rel(got, want) < (1e-13 if precision == "double" else 2e-5)
