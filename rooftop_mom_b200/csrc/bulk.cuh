@@ -58,7 +58,10 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, unsigned parity) {
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int* fault) {
     for (unsigned i = 0; i < kBulkWaitTries; ++i)
         if (mbar_test(bar, parity)) return true;
-    if (fault) atomicExch(fault, (int)RTM_ERR_TIMEOUT);
+    if (fault) {
+        *static_cast<volatile int*>(fault) = (int)RTM_ERR_TIMEOUT;  // pinned host memory; every writer writes this
+        __threadfence_system();
+    }
     return false;
 }
 

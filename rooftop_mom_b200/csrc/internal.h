@@ -164,10 +164,10 @@ void extracted_moments(double size_x, double size_y, double k, double out[7][4])
 
 int fast_fft_size(int count);
 
-// The device's fault word, which kernels with bounded waits set to RTM_ERR_TIMEOUT when a wait runs
-// out (a device variable: looking it up allocates nothing; the first lookup on a device loads its
-// module, so it is made outside any stream capture), and its check: reads and clears the word after
-// synchronising the stream, returning RTM_ERR_TIMEOUT if it was set.
+// The device's fault word, which kernels with bounded waits set to RTM_ERR_TIMEOUT when a wait runs out (pinned host
+// memory mapped by the devices; the first lookup of a process allocates it, so it is made outside any stream
+// capture), and its check: synchronises the stream, reads and clears the word, and returns RTM_ERR_TIMEOUT if it was
+// set.
 int device_fault_word(int** out);
 int device_fault_check(cudaStream_t s);
 
