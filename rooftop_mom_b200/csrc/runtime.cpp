@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdio>
 #include <algorithm>
+#include <chrono>
 #include <cstring>
 #include <complex>
 #include <map>
@@ -53,6 +54,34 @@ std::string format_bytes(double b) {
     return buf;
 }
 
+// The device's free memory as far as a request of `bytes` depends on it. cudaMemGetInfo takes 0.2 to 1 ms here (it
+// waits on the driver for all users of the machine) and every set-up and solve asks, so a reading decides requests of
+// up to a sixteenth of it for kReadingAge; larger requests and older readings read again. The library's own
+// allocations are taken off the reading. Called with g_budget_mu held.
+constexpr double kReadingAge = 0.1;  // seconds
+struct FreeReading {
+    double bytes = -1;
+    std::chrono::steady_clock::time_point at;
+};
+static FreeReading g_free[64];
+
+static bool free_memory(double bytes, double* out) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    FreeReading& r = g_free[dev & 63];
+    const auto now = std::chrono::steady_clock::now();
+    if (dev < 64 && r.bytes >= 16 * bytes && std::chrono::duration<double>(now - r.at).count() < kReadingAge) {
+        *out = r.bytes;
+        return true;
+    }
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
+    r.bytes = (double)free_b;
+    r.at = now;
+    *out = r.bytes;
+    return true;
+}
+
 int budget_require(double bytes, const char* what) {
     std::lock_guard<std::mutex> lk(g_budget_mu);
     if (g_ceiling > 0 && g_held + bytes > g_ceiling) {
@@ -60,10 +89,10 @@ int budget_require(double bytes, const char* what) {
                                             format_bytes(std::max(0.0, g_ceiling - g_held)) +
                                             " of the memory ceiling of " + format_bytes(g_ceiling) + " are left.");
     }
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes > (double)free_b) {
+    double free_b = 0;
+    if (free_memory(bytes, &free_b) && bytes > free_b) {
         return fail(RTM_ERR_OOM_BUDGET, std::string(what) + " needs " + format_bytes(bytes) + ", but only " +
-                                            format_bytes((double)free_b) + " are free on this device.");
+                                            format_bytes(free_b) + " are free on this device.");
     }
     return RTM_OK;
 }
@@ -129,6 +158,8 @@ int DeviceBuffer::alloc(size_t n) {
                                                 cudaGetErrorString(e));
         }
         capacity = cap;
+        std::lock_guard<std::mutex> lk(g_budget_mu);
+        g_free[device & 63].bytes -= (double)cap;
     }
     bytes = n;
     budget_hold((double)n);
