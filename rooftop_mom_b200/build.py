@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "librtm.so")
 OBJ = os.path.join(HERE, "_build")
-SOURCES = ["runtime.cpp", "capi.cpp", "server.cpp", "grid.cu", "grid_fast.cu", "assembly.cu", "krylov.cu", "ops.cu", "excitation.cu", "fixed_scratch.cu", "fault.cu", "tune.cpp", "batch.cu"]
+SOURCES = ["runtime.cpp", "capi.cpp", "server.cpp", "grid.cu", "grid_fast.cu", "assembly.cu", "krylov.cu", "strip_solve.cu", "ops.cu", "excitation.cu", "fixed_scratch.cu", "fault.cu", "tune.cpp", "batch.cu"]
 # sources compiled once for each form, so that their kernels compile side by side: object name -> (source, defines)
 FORMS = {f"grid_reg.{k}": ("grid_reg.cu", [f"-DRTM_REG_FORM={k}"]) for k in range(8)}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

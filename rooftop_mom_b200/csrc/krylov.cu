@@ -1121,6 +1121,9 @@ template <typename T>
 static int cocg(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* bv, const void* x0v, void* xv, int64_t n,
                 int nrhs, SolveResult& res, cudaStream_t s) {
     using T2 = typename Cx<T>::T2;
+    bool taken = false;
+    RTM_TRY(strip_cocg<T>(A, M, cfg, bv, x0v, xv, n, nrhs, res, s, &taken));
+    if (taken) return RTM_OK;
     const T2* b = static_cast<const T2*>(bv);
     const T2* x0 = static_cast<const T2*>(x0v);
     T2* x = static_cast<T2*>(xv);

@@ -36,6 +36,12 @@ struct SolveResult {
 int solve(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b, const void* x0, void* x, int64_t n, int nrhs,
           SolveResult& res, cudaStream_t s);
 
+// COCG of strip operators (both of them, or M null) in one kernel (strip_solve.cu), T their precision; *taken false, and
+// nothing done, for any other operator and for strips beyond a CTA's shared memory.
+template <typename T>
+int strip_cocg(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b, const void* x0, void* x, int64_t n,
+               int nrhs, SolveResult& res, cudaStream_t s, bool* taken);
+
 // FP64 outer iterative refinement around FP32 inner flexible GMRES (A64 FP64, A32 / M32 FP32). With
 // cfg.fallback_fp64, a refinement step that does not halve some right-hand side's FP64 residual (the FP32
 // inner solve diverged or stalled) ends the refinement, and the solve finishes in FP64 (A64 and M64, which

@@ -89,3 +89,57 @@ def test_circulants_of_any_face_count(grid, precision):
         want = S.fft_apply(rt, emb, rt.content, v[:rt.count])
         got = R.Operator(prob, product="fft", precision=precision).apply(v[:rt.count])
         assert rel(got, want) < (1e-13 if precision == "double" else 2e-5)
+
+
+@pytest.mark.parametrize("count", [(2, 1), (3, 1), (17, 1), (1, 40), (134, 1), (400, 1), (1, 701), (1600, 1)])
+@pytest.mark.parametrize("preconditioned", [True, False])
+def test_strip_solves(count, preconditioned):
+    """COCG on strips from the shortest to one that fits a CTA without the circulant alone, three right-hand sides at
+    once, one of them zero, and from an initial guess. The recurrence's history hangs on rounding past its first
+    iterations (the oracle's own moves by 0.5 % when b moves by 1e-15), so what is checked is what does not: the first
+    residuals, the iteration counts at 1e-6 (within 2, as for plates), and the residual of the returned current through
+    the oracle's product against the reported one."""
+    import numpy as np
+
+    from oracle import preconditioner as Q, solvers, spectra as S
+
+    R, prob, rt, gen = _setup(*count, a=0.05, b=0.05)
+    sub = S.subband_spectra(gen, rt.size_x, rt.size_y)
+    A = lambda v: S.split_apply(rt, sub, rt.content, v)  # noqa: E731
+    op, pc, M = R.Operator(prob, maxRhs=3), None, None
+    if preconditioned:
+        pc = R.Preconditioner(prob, kernel="rChan")
+        spec = Q.circulant(gen, rt.size_x, rt.size_y, kernel="rChan")
+        M = lambda v: S.fft_apply(rt, spec, rt.content, v)  # noqa: E731
+    n = rt.count
+    b = np.concatenate([random_vector(n, seed=1), np.zeros(n), random_vector(n, seed=2)])
+    limit = 60 if preconditioned or n == 1 else 3
+    solver = R.Solver("cg", tolerance=1e-6, maxIterationCount=limit)
+    got = solver.solve(op, b, preconditioner=pc, nrhs=3)
+    for k, r in enumerate(got):
+        part = b[k * n:(k + 1) * n]
+        if k == 1:
+            assert r.converged() and r.iterationCount() == 0 and not np.any(r.solution()) and r.residualNorm() == 0
+            continue
+        want = solvers.solve("cg", A, part, tol=1e-6, maxit=limit, precond=M)
+        assert r.converged() == want.converged and abs(r.iterationCount() - want.iteration_count) <= 2
+        assert len(r.residualNorms()) == r.iterationCount() + 1
+        assert np.allclose(r.residualNorms()[:3], want.residual_norms[:3], rtol=1e-9)
+        true = np.linalg.norm(part - A(r.solution())) / np.linalg.norm(part)
+        assert abs(r.residualNorm() - true) < 1e-10
+        assert not r.converged() or true < 1e-5
+    again = solver.solve(op, b[:n], preconditioner=pc, initialGuess=got[0].solution())
+    assert abs(again.residualNorms()[0] - got[0].residualNorm()) < 1e-10
+
+
+def test_a_strip_solve_of_more_iterations_than_one_launch():
+    """An unreachable tolerance runs to the iteration limit over several launches of the strip kernel."""
+    import numpy as np
+
+    R, prob, rt, gen = _setup(500, 1, a=0.05, b=0.05)
+    op = R.Operator(prob)
+    res = R.Solver("cg", tolerance=1e-300, maxIterationCount=1100).solve(op, random_vector(rt.count, seed=4))
+    assert not res.converged() and res.iterationCount() in range(1, 1101)
+    assert len(res.residualNorms()) == res.iterationCount() + 1
+    # the recurrence either ran out or broke down to a value that is not finite
+    assert res.iterationCount() == 1100 or not np.isfinite(res.residualNorms()[-1])
