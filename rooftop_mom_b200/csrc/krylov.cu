@@ -23,6 +23,7 @@
 
 #include "fft.cuh"
 #include "krylov.h"
+#include "pdl.cuh"
 
 namespace rtm {
 
@@ -92,6 +93,25 @@ __device__ __forceinline__ double2 cta_total(const double2* p, int nb) {
     return total;
 }
 
+// The rows of a CTA in COCG's kernels: kRowChunk consecutive ones where the launch has a CTA for every chunk (up to
+// 592 of them), a grid stride above. The chunks' sums then add in one order whatever n, so a plate in a batch (whose
+// vectors end in zeros up to the batch's stride) takes the same iterations to the last bit as alone.
+constexpr int kRowChunk = 2 * kRT;
+struct Rows {
+    int64_t first, end, step;
+    __device__ explicit Rows(int64_t n) {
+        if (n <= (int64_t)gridDim.x * kRowChunk) {
+            first = blockIdx.x * (int64_t)kRowChunk + threadIdx.x;
+            end = min(n, (blockIdx.x + (int64_t)1) * kRowChunk);
+            step = kRT;
+        } else {
+            first = blockIdx.x * (int64_t)kRT + threadIdx.x;
+            end = n;
+            step = (int64_t)gridDim.x * kRT;
+        }
+    }
+};
+
 // ============================================================================================
 // COCG
 struct CgState {
@@ -104,27 +124,40 @@ struct CgState {
     unsigned int counter;
 };
 
+// The CTA's two sums into its places of [2][gridDim.x] partials.
+__device__ __forceinline__ void cg_sums(double2 (&acc)[2], double2* part) {
+    __shared__ double2 both[2];
+    block_sum<2>(acc, both);
+    if (threadIdx.x < 2) part[threadIdx.x * gridDim.x + blockIdx.x] = both[threadIdx.x];
+}
+
+// plain: without a preconditioner z = r, so rho = r^T r is summed with the residual's norm (k_cg_update does the same),
+// and k_cg_rz is left out.
 template <typename T2>
 __global__ void __launch_bounds__(kRT) k_cg_start(const T2* __restrict__ b, const T2* __restrict__ r, int64_t n,
-                                                  CgState* st, double2* part, double* hist, int hist_stride) {
+                                                  CgState* st, double2* part, double* hist, int hist_stride, int plain) {
     const int rhs = blockIdx.y;
     const T2* br = b + rhs * n;
     const T2* rr = r + rhs * n;
-    double2 acc[1] = {make_double2(0, 0)};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double2 acc[2] = {make_double2(0, 0), make_double2(0, 0)};
+    const Rows rows(n);
+    for (int64_t i = rows.first; i < rows.end; i += rows.step) {
         const double2 bv = to_d2(br[i]), rv = to_d2(rr[i]);
         acc[0].x += bv.x * bv.x + bv.y * bv.y;
         acc[0].y += rv.x * rv.x + rv.y * rv.y;
+        if (plain) acc[1] = dadd(acc[1], dmul(rv, rv));
     }
-    double2* mine = part + ((int64_t)rhs * gridDim.x + blockIdx.x);
-    block_sum<1>(acc, mine);
+    double2* mine = part + (int64_t)rhs * 2 * gridDim.x;  // a CTA's two sums, each over the CTAs
+    cg_sums(acc, mine);
     if (!arrive(&st[rhs].counter)) return;
-    const double2 s = cta_total(part + (int64_t)rhs * gridDim.x, gridDim.x);
+    const double2 s = cta_total(mine, gridDim.x);
+    const double2 rho = plain ? cta_total(mine + gridDim.x, gridDim.x) : make_double2(0, 0);
     if (threadIdx.x == 0) {
         CgState& S = st[rhs];
         S.bnorm = sqrt(s.x);
         S.iteration = 0;
-        S.rho = S.beta = S.alpha = make_double2(0, 0);
+        S.beta = S.alpha = make_double2(0, 0);
+        S.rho = rho;
         if (S.bnorm == 0.0) {
             // IterativeMethod.m:53-56: the solution of a zero right-hand side is zero.
             S.zero_rhs = 1;
@@ -145,12 +178,14 @@ __global__ void __launch_bounds__(kRT) k_cg_start(const T2* __restrict__ b, cons
 template <typename T2>
 __global__ void __launch_bounds__(kRT) k_cg_rz(const T2* __restrict__ r, const T2* __restrict__ z, int64_t n,
                                                CgState* st, double2* part) {
+    griddep_wait();
     const int rhs = blockIdx.y;
     if (st[rhs].done) return;
     const T2* rr = r + rhs * n;
     const T2* zr = z + rhs * n;
     double2 acc[1] = {make_double2(0, 0)};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    const Rows rows(n);
+    for (int64_t i = rows.first; i < rows.end; i += rows.step)
         acc[0] = dadd(acc[0], dmul(to_d2(rr[i]), to_d2(zr[i])));
     block_sum<1>(acc, part + ((int64_t)rhs * gridDim.x + blockIdx.x));
     if (!arrive(&st[rhs].counter)) return;
@@ -166,6 +201,7 @@ __global__ void __launch_bounds__(kRT) k_cg_rz(const T2* __restrict__ r, const T
 template <typename T2>
 __global__ void __launch_bounds__(kRT) k_cg_dir(const T2* __restrict__ z, T2* __restrict__ d, int64_t n,
                                                 const CgState* st) {
+    griddep_wait();
     const int rhs = blockIdx.y;
     const CgState& S = st[rhs];
     if (S.done) return;
@@ -173,7 +209,8 @@ __global__ void __launch_bounds__(kRT) k_cg_dir(const T2* __restrict__ z, T2* __
     T2* dr = d + rhs * n;
     const bool first = S.iteration == 0;
     const double2 beta = S.beta;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const Rows rows(n);
+    for (int64_t i = rows.first; i < rows.end; i += rows.step) {
         const double2 zv = to_d2(zr[i]);
         dr[i] = first ? zr[i] : from_d2<T2>(dadd(zv, dmul(beta, to_d2(dr[i]))));
     }
@@ -183,12 +220,14 @@ __global__ void __launch_bounds__(kRT) k_cg_dir(const T2* __restrict__ z, T2* __
 template <typename T2>
 __global__ void __launch_bounds__(kRT) k_cg_dq(const T2* __restrict__ d, const T2* __restrict__ q, int64_t n,
                                                CgState* st, double2* part) {
+    griddep_wait();
     const int rhs = blockIdx.y;
     if (st[rhs].done) return;
     const T2* dr = d + rhs * n;
     const T2* qr = q + rhs * n;
     double2 acc[1] = {make_double2(0, 0)};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    const Rows rows(n);
+    for (int64_t i = rows.first; i < rows.end; i += rows.step)
         acc[0] = dadd(acc[0], dmul(to_d2(dr[i]), to_d2(qr[i])));
     block_sum<1>(acc, part + ((int64_t)rhs * gridDim.x + blockIdx.x));
     if (!arrive(&st[rhs].counter)) return;
@@ -200,7 +239,8 @@ __global__ void __launch_bounds__(kRT) k_cg_dq(const T2* __restrict__ d, const T
 template <typename T2>
 __global__ void __launch_bounds__(kRT) k_cg_update(T2* __restrict__ x, T2* __restrict__ r, const T2* __restrict__ d,
                                                    const T2* __restrict__ q, int64_t n, CgState* st, double2* part,
-                                                   double* hist, int hist_stride) {
+                                                   double* hist, int hist_stride, int plain) {
+    griddep_wait();
     const int rhs = blockIdx.y;
     if (st[rhs].done) return;
     const double2 alpha = st[rhs].alpha;
@@ -208,8 +248,9 @@ __global__ void __launch_bounds__(kRT) k_cg_update(T2* __restrict__ x, T2* __res
     T2* rr = r + rhs * n;
     const T2* dr = d + rhs * n;
     const T2* qr = q + rhs * n;
-    double2 acc[1] = {make_double2(0, 0)};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double2 acc[2] = {make_double2(0, 0), make_double2(0, 0)};
+    const Rows rows(n);
+    for (int64_t i = rows.first; i < rows.end; i += rows.step) {
         const double2 xv = dadd(to_d2(xr[i]), dmul(alpha, to_d2(dr[i])));
         const double2 aq = dmul(alpha, to_d2(qr[i]));
         const double2 rv0 = to_d2(rr[i]);
@@ -219,12 +260,19 @@ __global__ void __launch_bounds__(kRT) k_cg_update(T2* __restrict__ x, T2* __res
         rr[i] = rs;
         const double2 rd = to_d2(rs);
         acc[0].x += rd.x * rd.x + rd.y * rd.y;
+        if (plain) acc[1] = dadd(acc[1], dmul(rd, rd));
     }
-    block_sum<1>(acc, part + ((int64_t)rhs * gridDim.x + blockIdx.x));
+    double2* mine = part + (int64_t)rhs * 2 * gridDim.x;
+    cg_sums(acc, mine);
     if (!arrive(&st[rhs].counter)) return;
-    const double s = cta_total(part + (int64_t)rhs * gridDim.x, gridDim.x).x;
+    const double s = cta_total(mine, gridDim.x).x;
+    const double2 rho = plain ? cta_total(mine + gridDim.x, gridDim.x) : make_double2(0, 0);
     if (threadIdx.x == 0) {
         CgState& S = st[rhs];
+        if (plain) {
+            S.beta = ddiv(rho, S.rho);
+            S.rho = rho;
+        }
         S.iteration += 1;
         const double h = sqrt(s) / S.bnorm;
         hist[(int64_t)rhs * hist_stride + S.iteration] = h;
@@ -250,6 +298,7 @@ struct GmState {
     int cycle_ran;
     int skip_update;  // = !cycle_ran: the preconditioner's skip flag for the right-preconditioned update
     unsigned int counter;
+    unsigned int bar, bar_base;  // k_gm_arnoldi: its barrier's arrivals, and their count before this step
 };
 
 struct GmArrays {
@@ -330,27 +379,13 @@ __global__ void __launch_bounds__(kRT) k_gm_v0(const T2* __restrict__ w, T2* __r
     }
 }
 
-// The rest of an Arnoldi step once ||w|| is known: the Hessenberg column, its previous rotations,
-// the new rotation, the rotated right-hand side, the history and the stopping tests (one thread).
-// col, cs, sn: the Hessenberg column being formed and the rotations, in global memory or staged in
-// shared memory by the caller with col already holding h (the rotation chain is sequential; staged, each
-// step costs a shared-memory access instead of a global one).
-__device__ void arnoldi_finish(GmState& S, GmArrays& ar, int rhs, double s, double2* col, double2* cs, double2* sn,
-                               bool staged) {
+// The end of an Arnoldi step: the Hessenberg column col (its previous rotations applied) with the subdiagonal
+// ||w|| = sqrt(s), the new rotation, the rotated right-hand side, the history and the stopping tests (one thread).
+__device__ void arnoldi_rotate(GmState& S, GmArrays& ar, int rhs, double s, double2* col, double2* cs, double2* sn) {
     const double sub = sqrt(s);
     const int m = ar.m, j = S.step;
     double2* g = ar.g + (int64_t)rhs * (m + 1);
-    const double2* h = ar.h + (int64_t)rhs * (m + 1);
-    if (!staged)
-        for (int k = 0; k <= j; ++k) col[k] = h[k];
     col[j + 1] = make_double2(sub, 0);
-    for (int k = 0; k < j; ++k) {
-        const double2 a0 = col[k], a1 = col[k + 1];
-        col[k] = dadd(dmulc(cs[k], a0), dmulc(sn[k], a1));
-        const double2 t = dmul(sn[k], a0);
-        const double2 u = dmul(cs[k], a1);
-        col[k + 1] = make_double2(u.x - t.x, u.y - t.y);
-    }
     // generateRotation_.m:11-18
     const double2 a = col[j], bsub = col[j + 1];
     const double radius = sqrt(a.x * a.x + a.y * a.y + bsub.x * bsub.x + bsub.y * bsub.y);
@@ -380,6 +415,26 @@ __device__ void arnoldi_finish(GmState& S, GmArrays& ar, int rhs, double s, doub
     S.done = S.converged || S.iteration >= S.max_iterations;
 }
 
+// The rest of an Arnoldi step once ||w|| is known: the Hessenberg column, its previous rotations,
+// the new rotation, the rotated right-hand side, the history and the stopping tests (one thread).
+// col, cs, sn: the Hessenberg column being formed and the rotations, in global memory or staged in
+// shared memory by the caller with col already holding h (the rotation chain is sequential; staged, each
+// step costs a shared-memory access instead of a global one).
+__device__ void arnoldi_finish(GmState& S, GmArrays& ar, int rhs, double s, double2* col, double2* cs, double2* sn,
+                               bool staged) {
+    const int m = ar.m, j = S.step;
+    const double2* h = ar.h + (int64_t)rhs * (m + 1);
+    if (!staged)
+        for (int k = 0; k <= j; ++k) col[k] = h[k];
+    for (int k = 0; k < j; ++k) {
+        const double2 a0 = col[k], a1 = col[k + 1];
+        col[k] = dadd(dmulc(cs[k], a0), dmulc(sn[k], a1));
+        const double2 t = dmul(sn[k], a0);
+        const double2 u = dmul(cs[k], a1);
+        col[k + 1] = make_double2(u.x - t.x, u.y - t.y);
+    }
+    arnoldi_rotate(S, ar, rhs, s, col, cs, sn);
+}
 // Asynchronous global -> shared copies (cp.async, sm_80 and later): a thread issues all the copies
 // of a tile without waiting, then waits for its groups before the CTA barrier.
 template <int BYTES> __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
@@ -867,6 +922,362 @@ template <typename T2> static void launch_orth(const T2* V, T2* w, int64_t n, in
     count_launch();
 }
 
+// --------------------------------------------------------------------------------------------
+// A whole Arnoldi step's orthogonalisation in one cooperative launch, for bases of up to kStreamCols columns whose
+// rows, split over the CTAs the device holds at once, make chunks of at most kArnoldiRows: the passes of
+// k_gm_orth_stream, the norm, the Hessenberg column and V[:, step + 1] = w / ||w||. The CTAs of a right-hand side
+// meet at two barriers; every CTA then sums the per-CTA partials itself, in one order. The norm needs no third one: the
+// last correction c is orthogonal to what it leaves, so ||w - V c||^2 = ||w||^2 - ||c||^2 with ||w||^2 summed beside c.
+// That loses nothing while c is small, as a second projection's is (rounding of the first); where ||c||^2 is above
+// kArnLeft of ||w||^2 (a second pass after heavy cancellation, or one pass alone) the norm is summed after all. A CTA keeps its chunk of w in shared memory from the first pass to the last, and as many of the basis
+// columns as fit beside it, so that these are read once instead of four times. One more CTA per right-hand side
+// holds no rows: it runs the rotations of the new Hessenberg column while the others subtract the last projection.
+//
+// Bound: the basis's L2 bandwidth and three barriers. 256 x 256 faces, one right-hand side, 100 iterations: the three
+// passes and k_gm_next took 46 us a step, four launches each waiting for the slowest CTA's chain of loads and sums.
+constexpr int kArnThreads = 512, kArnWarps = kArnThreads / 32, kArnCols = kStreamCols / kArnWarps;
+constexpr int kArnParts = 2 * kStreamCols + 2;  // partials a CTA
+constexpr int kArnoldiRows = 2048;
+constexpr size_t kArnSmem = 216 * 1024;  // dynamic shared memory (about 7 KB more are static)
+constexpr double kArnLeft = 1e-6;  // the subtraction's relative error then stays below 1e-6 of its terms' rounding
+constexpr unsigned kArnPolls = 1u << 21;  // of a barrier, about 0.7 us each
+
+__device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Waits until `target` arrivals (modulo 2^32) have been counted; false, with the fault word set, when they have not
+// within kArnPolls polls.
+__device__ __forceinline__ bool arnoldi_barrier(unsigned* bar, unsigned target, int* fault) {
+    __shared__ int met;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        // release and acquire at the device's scope order what the CTA wrote before and reads after
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(bar) : "memory");
+        met = 0;
+        for (unsigned i = 0; i < kArnPolls; ++i)
+            if ((int)(load_acquire(bar) - target) >= 0) {
+                met = 1;
+                break;
+            }
+        if (!met && fault) *static_cast<volatile int*>(fault) = (int)RTM_ERR_TIMEOUT;
+    }
+    __syncthreads();
+    return met != 0;
+}
+
+// The dots of this warp's columns k0 + kArnWarps c (c < C, below cols) with the chunk ws over the rows [rs, re), U
+// rows a lane and column in flight. Columns below `cached` come from shared memory (Vs, leading dimension ld), or go
+// there when `fill` is set. Products in the basis's precision, sums in FP64.
+template <typename T2, int C, int U>
+__device__ __forceinline__ void arnoldi_dots(const T2* __restrict__ V, int64_t col, const T2* ws, T2* Vs, int ld,
+                                             int cached, bool fill, int k0, int cols, int rs, int re,
+                                             double2 (&acc)[kArnCols]) {
+    const T2 zero = from_d2<T2>(make_double2(0, 0));
+    for (int r0 = rs + (int)(threadIdx.x & 31); r0 < re; r0 += 32 * U) {
+        T2 t[C][U], x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = r0 + 32 * u;
+            const bool in = r < re;
+            x[u] = in ? ws[r] : zero;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int k = k0 + kArnWarps * c;
+                const bool use = in && k < cols;
+                if (!fill && k < cached) t[c][u] = use ? Vs[k * ld + r] : zero;
+                else t[c][u] = use ? __ldg(&V[k * col + r]) : zero;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = r0 + 32 * u;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int k = k0 + kArnWarps * c;
+                if (fill && r < re && k < cols && k < cached) Vs[k * ld + r] = t[c][u];
+                const double2 p = to_d2(amulc(t[c][u], x[u]));
+                acc[c].x += p.x;
+                acc[c].y += p.y;
+            }
+        }
+    }
+}
+
+// V: the basis [m + 1][nrhs][n], read up to column `step` and written at column step + 1 (vnext: the same memory).
+template <typename T2>
+__global__ void __launch_bounds__(kArnThreads, 1)
+    k_gm_arnoldi(const T2* __restrict__ V, T2* vnext, const T2* __restrict__ w, int64_t n, int nrhs, GmState* st, GmArrays ar,
+                 double2* parts, int passes, int chunk, int room, int* fault) {
+    using A2 = typename OrthAcc<T2>::type;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double2 sum_h[kStreamCols], sum_c[kStreamCols], red[kStreamCols];
+    __shared__ A2 coef[kStreamCols];
+    __shared__ double2 scol[kStreamCols + 1], scs[kStreamCols], ssn[kStreamCols];
+    __shared__ double total;
+    const int rhs = blockIdx.y, B = gridDim.x - 1, blk = blockIdx.x;
+    GmState& S = st[rhs];
+    if (!S.active) return;
+    const int j = S.step, cols = j + 1, m = ar.m;
+    const unsigned base = S.bar_base, all = gridDim.x;
+    const bool scalar = blk == B;
+    const int64_t c0 = (int64_t)blk * chunk;
+    const int len = scalar ? 0 : (int)(n - c0 < (int64_t)chunk ? n - c0 : (int64_t)chunk);
+    T2* ws = reinterpret_cast<T2*>(smem_raw);
+    T2* Vs = ws + chunk;
+    const int cached = room < cols ? room : cols;
+    const int64_t col = (int64_t)nrhs * n;
+    const T2* Vr = V + (int64_t)rhs * n + c0;
+    double2* part = parts + (int64_t)rhs * kArnParts * B;  // [pass][column][CTA], then two norms' [CTA]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+    auto dots = [&](int pass) {
+        const bool wide = cols >= kArnWarps;
+        const int slices = wide ? 1 : kArnWarps / cols;
+        const int k0 = wide ? warp : warp % cols, slice = wide ? 0 : warp / cols;
+        double2 acc[kArnCols];
+#pragma unroll
+        for (int c = 0; c < kArnCols; ++c) acc[c] = make_double2(0, 0);
+        const bool fill = pass == 0;
+        if (!wide) {
+            if (slice < slices)
+                arnoldi_dots<T2, 1, 8>(Vr, col, ws, Vs, chunk, cached, fill, k0, cols, (int)((int64_t)len * slice / slices),
+                                       (int)((int64_t)len * (slice + 1) / slices), acc);
+        } else if (cols <= 2 * kArnWarps) {
+            arnoldi_dots<T2, 2, 8>(Vr, col, ws, Vs, chunk, cached, fill, k0, cols, 0, len, acc);
+        } else {
+            arnoldi_dots<T2, kArnCols, 4>(Vr, col, ws, Vs, chunk, cached, fill, k0, cols, 0, len, acc);
+        }
+#pragma unroll
+        for (int c = 0; c < kArnCols; ++c) {
+            double2 v = acc[c];
+            for (int o = 16; o > 0; o >>= 1) {
+                v.x += __shfl_down_sync(0xffffffffu, v.x, o);
+                v.y += __shfl_down_sync(0xffffffffu, v.y, o);
+            }
+            // wide: column warp + 16 c; else the slices of a column at column + cols slice (< 16)
+            if (lane == 0 && (wide || c == 0)) red[warp + kArnWarps * c] = v;
+        }
+        __syncthreads();
+        if (tid < cols) {
+            double2 v = red[tid];
+            if (!wide)
+                for (int g = 1; g < slices; ++g) v = dadd(v, red[tid + g * cols]);
+            part[((int64_t)pass * kStreamCols + tid) * B + blk] = v;
+        }
+    };
+    // every CTA's sum of a pass's partials, a warp a column
+    auto gather = [&](int pass, double2* out) {
+        for (int k = warp; k < cols; k += kArnWarps) {
+            const double2* p = part + ((int64_t)pass * kStreamCols + k) * B;
+            double2 v = make_double2(0, 0);
+            for (int b = lane; b < B; b += 32) v = dadd(v, __ldcg(&p[b]));
+            for (int o = 16; o > 0; o >>= 1) {
+                v.x += __shfl_down_sync(0xffffffffu, v.x, o);
+                v.y += __shfl_down_sync(0xffffffffu, v.y, o);
+            }
+            if (lane == 0) {
+                out[k] = v;
+                coef[k] = from_d2<A2>(v);
+            }
+        }
+        __syncthreads();
+    };
+    // w -= V coef over the chunk; returns this thread's part of ||w||^2
+    auto subtract = [&]() {
+        double nrm = 0;
+        for (int r = tid; r < len; r += kArnThreads) {
+            A2 v = ws[r];
+            int k = 0;
+            for (; k < cached; ++k) {
+                const A2 p = amul(Vs[k * chunk + r], coef[k]);
+                v.x -= p.x;
+                v.y -= p.y;
+            }
+            constexpr int UB = 8;
+            for (; k + UB <= cols; k += UB) {
+                T2 t[UB];
+#pragma unroll
+                for (int u = 0; u < UB; ++u) t[u] = __ldg(&Vr[(k + u) * col + r]);
+#pragma unroll
+                for (int u = 0; u < UB; ++u) {
+                    const A2 p = amul(t[u], coef[k + u]);
+                    v.x -= p.x;
+                    v.y -= p.y;
+                }
+            }
+            for (; k < cols; ++k) {
+                const A2 p = amul(__ldg(&Vr[k * col + r]), coef[k]);
+                v.x -= p.x;
+                v.y -= p.y;
+            }
+            ws[r] = v;
+            const double2 d = to_d2(v);
+            nrm += d.x * d.x + d.y * d.y;
+        }
+        return nrm;
+    };
+
+    // the CTA's sum of v (warps, then the warps' sums in order) as its partial of the norm
+    auto put_norm = [&](int slot, double v) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) red[warp].x = v;
+        __syncthreads();
+        if (tid == 0) {
+            double sum = 0;
+            for (int q = 0; q < kArnWarps; ++q) sum += red[q].x;
+            part[(int64_t)(2 * kStreamCols + slot) * B + blk] = make_double2(sum, 0);
+        }
+        __syncthreads();
+    };
+    auto gather_norm = [&](int slot) {
+        if (warp == 0) {
+            double v = 0;
+            for (int b = lane; b < B; b += 32) v += __ldcg(&part[(int64_t)(2 * kStreamCols + slot) * B + b]).x;
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) total = v;
+        }
+        __syncthreads();
+    };
+    double left = 0;
+    if (tid == 0) total = 0;
+    for (int r = tid; r < len; r += kArnThreads) ws[r] = w[(int64_t)rhs * n + c0 + r];
+    __syncthreads();
+    if (!scalar) dots(0);
+    unsigned at = base + all;
+    bool met = arnoldi_barrier(&S.bar, at, fault);
+    if (met) {
+        gather(0, sum_h);
+        if (passes == 2) {
+            if (!scalar) {
+                put_norm(0, subtract());
+                dots(1);
+            }
+            at += all;
+            met = arnoldi_barrier(&S.bar, at, fault);
+            if (met) {
+                gather(1, sum_c);
+                gather_norm(0);
+                for (int k = 0; k < cols; ++k) left += sum_c[k].x * sum_c[k].x + sum_c[k].y * sum_c[k].y;
+            }
+        }
+    }
+    // every CTA reads the same sums, so all take the same way
+    const bool again = !(passes == 2 && met && left <= kArnLeft * total);
+    double sub2 = again ? 0.0 : total - left;
+    if (met) {
+        if (!scalar) {
+            const double own = subtract();
+            if (again) put_norm(1, own);
+        } else {
+            // the new column's previous rotations (the chain is sequential: staged in shared memory)
+            const double2* cs = ar.cs + (int64_t)rhs * m;
+            const double2* sn = ar.sn + (int64_t)rhs * m;
+            for (int k = tid; k < cols; k += kArnThreads) {
+                scol[k] = passes == 2 ? dadd(sum_h[k], sum_c[k]) : sum_h[k];
+                if (k < j) {
+                    scs[k] = cs[k];
+                    ssn[k] = sn[k];
+                }
+            }
+            __syncthreads();
+            if (tid == 0) {
+                double2 a0 = scol[0];
+                for (int k = 0; k < j; ++k) {
+                    const double2 a1 = scol[k + 1];
+                    scol[k] = dadd(dmulc(scs[k], a0), dmulc(ssn[k], a1));
+                    const double2 t = dmul(ssn[k], a0), u = dmul(scs[k], a1);
+                    a0 = make_double2(u.x - t.x, u.y - t.y);
+                }
+                scol[j] = a0;
+            }
+        }
+        if (again) {
+            at += all;
+            met = arnoldi_barrier(&S.bar, at, fault);
+            if (met) {
+                gather_norm(1);
+                sub2 = total;
+            }
+        }
+    }
+    if (!met) {
+        // a barrier ran out: this right-hand side stops (the host reports the fault word)
+        if (scalar && tid == 0) {
+            S.active = 0;
+            S.skip_step = 1;
+            S.done = 1;
+        }
+        return;
+    }
+    if (!scalar) {
+        const double sub = sqrt(sub2), inv = sub != 0 ? 1.0 / sub : 0.0;
+        T2* out = vnext + ((int64_t)(j + 1) * nrhs + rhs) * n + c0;
+        for (int r = tid; r < len; r += kArnThreads) {
+            const double2 v = to_d2(ws[r]);
+            out[r] = from_d2<T2>(make_double2(v.x * inv, v.y * inv));
+        }
+        return;
+    }
+    __syncthreads();  // scol
+    if (tid == 0) {
+        S.bar_base = at;
+        arnoldi_rotate(S, ar, rhs, sub2, scol, ar.cs + (int64_t)rhs * m, ar.sn + (int64_t)rhs * m);
+    }
+    __syncthreads();
+    double2* column = ar.H + ((int64_t)rhs * m + j) * (m + 1);
+    for (int k = tid; k <= j + 1; k += kArnThreads) column[k] = scol[k];
+}
+
+// How k_gm_arnoldi runs for nrhs vectors of n rows on the current device: CTAs with rows per right-hand side, rows a
+// CTA, basis columns kept in shared memory. False where the general passes serve: longer bases, chunks above
+// kArnoldiRows, more right-hand sides than the device holds CTAs for.
+struct ArnoldiShape {
+    int blocks = 0, chunk = 0, room = 0;
+    size_t smem = 0;
+};
+template <typename T2> static bool arnoldi_shape(int64_t n, int nrhs, int m, ArnoldiShape* out) {
+    if (m + 1 > kStreamCols) return false;
+    int dev = 0, sms = 0, coop = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
+        return false;
+    const int64_t per = sms / nrhs - 1;  // one CTA an SM, one of them without rows
+    if (per < 1) return false;
+    // at least 128 rows a CTA: below, its share costs less than the partials it adds
+    const int64_t want = std::min<int64_t>(per, (n + 127) / 128);
+    const int64_t chunk = ((n + want - 1) / want + 31) / 32 * 32;
+    if (chunk > kArnoldiRows) return false;
+    out->chunk = (int)chunk;
+    out->blocks = (int)((n + chunk - 1) / chunk);
+    const size_t column = (size_t)chunk * sizeof(T2);
+    out->room = (int)std::min<size_t>(m, (kArnSmem - column) / column);
+    out->smem = column * (1 + out->room);
+    return true;
+}
+
+template <typename T2>
+static int launch_arnoldi(const ArnoldiShape& a, T2* V, const T2* w, int64_t n, int nrhs, GmState* st, const GmArrays& ar,
+                          double2* parts, int passes, int* fault, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.blocks + 1, nrhs);
+    cfg.blockDim = dim3(kArnThreads);
+    cfg.dynamicSmemBytes = a.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    RTM_CUDA(cudaLaunchKernelEx(&cfg, k_gm_arnoldi<T2>, (const T2*)V, V, w, n, nrhs, st, ar, parts, passes, a.chunk, a.room,
+                                fault));
+    count_launch();
+    return RTM_OK;
+}
+
 // V[:, step] = w / H(step, step - 1) while the cycle goes on.
 template <typename T2>
 __global__ void __launch_bounds__(kRT) k_gm_next(const T2* __restrict__ w, T2* __restrict__ V, int64_t n, int nrhs,
@@ -1136,7 +1547,7 @@ static int cocg(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* bv
     RTM_TRY(d.alloc(vec));
     RTM_TRY(q.alloc(vec));
     RTM_TRY(stb.alloc(sizeof(CgState) * nrhs));
-    RTM_TRY(part.alloc(sizeof(double2) * nb * nrhs));
+    RTM_TRY(part.alloc(sizeof(double2) * 2 * nb * nrhs));
     const int hs = cfg.max_iterations + 1;
     RTM_TRY(hist.alloc(sizeof(double) * hs * nrhs));
     RTM_TRY(resb.alloc(sizeof(double2) * nrhs));
@@ -1166,7 +1577,8 @@ static int cocg(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* bv
         RTM_CUDA(cudaMemsetAsync(x, 0, vec, s));
         RTM_CUDA(cudaMemcpyAsync(r.ptr, b, vec, cudaMemcpyDeviceToDevice, s));
     }
-    k_cg_start<T2><<<grid, kRT, 0, s>>>(b, r.as<T2>(), n, st, part.as<double2>(), hist.as<double>(), hs);
+    const int plain = M ? 0 : 1;
+    k_cg_start<T2><<<grid, kRT, 0, s>>>(b, r.as<T2>(), n, st, part.as<double2>(), hist.as<double>(), hs, plain);
     count_launch();
     T2* zp = M ? z.as<T2>() : r.as<T2>();
     const int every = cfg.check_every > 0 ? cfg.check_every : 16;
@@ -1176,14 +1588,19 @@ static int cocg(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* bv
     // `every` iterations as one graph; iterations past the stopping test are no-ops on the device.
     auto chunk_body = [&]() -> int {
         for (int it = 0; it < every; ++it) {
-            if (M) RTM_TRY(M->apply(r.ptr, z.ptr, nrhs, s, skip));
-            k_cg_rz<T2><<<grid, kRT, 0, s>>>(r.as<T2>(), zp, n, st, part.as<double2>());
-            k_cg_dir<T2><<<grid, kRT, 0, s>>>(zp, d.as<T2>(), n, st);
+            if (M) {
+                RTM_TRY(M->apply(r.ptr, z.ptr, nrhs, s, skip));
+                RTM_CUDA(launch_dependent(k_cg_rz<T2>, grid, dim3(kRT), 0, s, (const T2*)r.as<T2>(), (const T2*)zp, n, st,
+                                          part.as<double2>()));
+                count_launch();
+            }
+            RTM_CUDA(launch_dependent(k_cg_dir<T2>, grid, dim3(kRT), 0, s, (const T2*)zp, d.as<T2>(), n, (const CgState*)st));
             RTM_TRY(A->apply(d.ptr, q.ptr, nrhs, s, skip));
-            k_cg_dq<T2><<<grid, kRT, 0, s>>>(d.as<T2>(), q.as<T2>(), n, st, part.as<double2>());
-            k_cg_update<T2><<<grid, kRT, 0, s>>>(x, r.as<T2>(), d.as<T2>(), q.as<T2>(), n, st, part.as<double2>(),
-                                                 hist.as<double>(), hs);
-            count_launch(4);
+            RTM_CUDA(launch_dependent(k_cg_dq<T2>, grid, dim3(kRT), 0, s, (const T2*)d.as<T2>(), (const T2*)q.as<T2>(), n, st,
+                                      part.as<double2>()));
+            RTM_CUDA(launch_dependent(k_cg_update<T2>, grid, dim3(kRT), 0, s, x, r.as<T2>(), (const T2*)d.as<T2>(),
+                                      (const T2*)q.as<T2>(), n, st, part.as<double2>(), hist.as<double>(), hs, plain));
+            count_launch(3);
         }
         RTM_CUDA(cudaGetLastError());
         return RTM_OK;
@@ -1311,6 +1728,16 @@ static int gmres(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b
     k_gm_norm<T2><<<grid, kRT, 0, s>>>(w.as<T2>(), n, st, ar, 1, 1);
     count_launch();
     // function attributes are set before the capture
+    ArnoldiShape shape;
+    DeviceBuffer parts;
+    StreamSyncGuard parts_guard(s);
+    const bool fused = arnoldi_shape<T2>(n, nrhs, m, &shape);
+    int* fault = nullptr;
+    if (fused) {
+        RTM_TRY(device_fault_word(&fault));
+        RTM_TRY(parts.alloc(sizeof(double2) * kArnParts * (size_t)shape.blocks * nrhs));
+        RTM_CUDA(cudaFuncSetAttribute(k_gm_arnoldi<T2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kArnSmem));
+    }
     RTM_CUDA(cudaFuncSetAttribute(k_gm_orth<T2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrthSmemMax));
     {
         int sb, sc;
@@ -1336,6 +1763,11 @@ static int gmres(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b
                 RTM_TRY(M->apply(t.ptr, w.ptr, nrhs, s, skip_step));
             } else {
                 RTM_TRY(A->apply(vj, w.ptr, nrhs, s, skip_step));
+            }
+            if (fused) {
+                RTM_TRY(launch_arnoldi<T2>(shape, Vp, w.as<T2>(), n, nrhs, st, ar, parts.as<double2>(),
+                                           cfg.gram_schmidt_passes == 1 ? 1 : 2, fault, s));
+                continue;
             }
             // CGS2: project (mode 0), subtract and project again (1), subtract the correction and take the
             // norm (2). One pass skips mode 1: mode 2 then subtracts the first projection, which mode 0

@@ -1,10 +1,15 @@
-// Programmatic dependent launch (sm_90 and later), used inside the three kernels of a power-of-two product
-// (the x-mix and the y-inverse are launched as dependents): a kernel launched with the programmatic
-// stream-serialisation attribute may be scheduled while its predecessor on the stream is still running;
-// its CTAs then block in griddep_wait() until the predecessor has completed and its memory is visible.
-// Each kernel launched this way calls griddep_wait() before anything else (so it reads no data of its
-// predecessor early) and griddep_launch_dependents() right after, so that its own successor may be
-// scheduled as its CTAs retire. Outside such a launch both instructions do nothing.
+// Programmatic dependent launch (sm_90 and later), used by the kernels of products, preconditioner applies and COCG
+// iterations: a kernel launched with the programmatic stream-serialisation attribute is set up while its predecessor on
+// the stream is still running; its CTAs then block in griddep_wait() until the predecessor has completed and its memory
+// is visible. Each kernel launched this way calls griddep_wait() before anything else, so it reads no data of its
+// predecessor early (nor of that one's predecessors, which completed before it). After a predecessor that is a copy, or
+// outside such a launch, the wait is the ordinary one or none.
+//
+// griddep_launch_dependents() lets a kernel's dependents start once all its CTAs have called it. Only the passes of
+// grid_reg.cu do: their long straight code then starts to load behind the predecessor (a 64 x 64 circulant apply: 8.4 us
+// against 10.1 without). Elsewhere the dependents' CTAs would fill the SMs whose CTAs end first, several on one SM, and
+// run the slower for it (a 256 x 256 product after a block-Jacobi apply that did so: 24 us instead of 19; the FP32
+// 512 x 512 product 39 instead of 35).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -143,3 +143,51 @@ def test_a_strip_solve_of_more_iterations_than_one_launch():
     assert len(res.residualNorms()) == res.iterationCount() + 1
     # the recurrence either ran out or broke down to a value that is not finite
     assert res.iterationCount() == 1100 or not np.isfinite(res.residualNorms()[-1])
+
+
+def _gmres_case(n, seed, nrhs):
+    import numpy as np
+
+    rng = np.random.default_rng(seed)
+    A = np.eye(n) + 0.4 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / math.sqrt(2 * n)
+    return A, random_vector(n * nrhs, seed=seed + 1)
+
+
+@pytest.mark.parametrize("n,restart,nrhs", [(1, 1, 1), (2, 5, 1), (31, 15, 2), (33, 16, 3), (129, 17, 1), (130, 32, 5),
+                                            (257, 33, 1), (300, 63, 1), (300, 64, 1), (700, 50, 2), (40, 20, 75)])
+@pytest.mark.parametrize("passes", [2, 1])
+def test_arnoldi_steps(n, restart, nrhs, passes):
+    """GMRES over bases from one column to the longest of the one-launch Arnoldi step (63) and one beyond it, rows from
+    one to several CTAs, and right-hand sides from one to more than a device's CTAs: the oracle's residual histories
+    (its orthogonalisation is backward stable, so they agree to a few roundings: 1e-8) and solutions."""
+    import numpy as np
+
+    import rooftop_mom_b200 as R
+    from oracle import solvers
+
+    A, b = _gmres_case(n, 11, nrhs)
+    solver = R.Solver("gmres", tolerance=1e-10, maxIterationCount=90, restart=restart, gramSchmidtPasses=passes)
+    got = solver.solve(R.DenseOperator(A), b, nrhs=nrhs)
+    for k, r in enumerate(got if nrhs > 1 else [got]):
+        want = solvers.solve("gmres", A, b[k * n:(k + 1) * n], tol=1e-10, maxit=90, restart=restart)
+        assert r.converged() == want.converged and abs(r.iterationCount() - want.iteration_count) <= 1
+        h = min(r.iterationCount(), want.iteration_count) + 1
+        assert np.allclose(r.residualNorms()[:h], want.residual_norms[:h], rtol=1e-8, atol=1e-13)
+        assert rel(r.solution(), want.solution) < 1e-8
+
+
+def test_arnoldi_steps_whose_basis_spans_the_solution():
+    """A matrix whose Krylov space ends after three steps: the second projection removes all there is, so the norm is
+    summed rather than subtracted, and the solve ends there."""
+    import numpy as np
+
+    import rooftop_mom_b200 as R
+
+    n = 500
+    rng = np.random.default_rng(5)
+    u = np.linalg.qr(rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2)))[0]
+    A = np.eye(n) + u @ np.diag([2.0, 5.0j]) @ u.conj().T
+    b = random_vector(n, seed=9)
+    res = R.Solver("gmres", tolerance=1e-12, maxIterationCount=40, restart=20).solve(R.DenseOperator(A), b)
+    assert res.converged() and res.iterationCount() == 3
+    assert rel(A @ res.solution(), b) < 1e-12
