@@ -2,6 +2,7 @@
 #include <algorithm>
 
 #include "batch.h"
+#include "pdl.cuh"
 
 namespace rtm {
 namespace {
@@ -9,6 +10,7 @@ namespace {
 template <typename T2>
 __global__ void k_zero_tails(T2* __restrict__ y, int64_t stride, const int64_t* __restrict__ counts, const int* skip,
                              int skip_stride) {
+    griddep_wait();
     const int k = blockIdx.y;
     if (skip && skip[(int64_t)k * skip_stride]) return;
     T2* yk = y + (int64_t)k * stride;
@@ -25,11 +27,11 @@ int zero_tails(void* y, int precision, int64_t stride, const int64_t* counts_dev
     // about eight elements a thread: a CTA or a few per entry
     const dim3 grid((unsigned)std::min<int64_t>(64, (max_tail + 2047) / 2048), count);
     if (precision == RTM_FP64)
-        k_zero_tails<double2><<<grid, 256, 0, s>>>(static_cast<double2*>(y), stride, counts_device, skip.ptr,
-                                                   skip.stride);
+        RTM_CUDA(launch_dependent(k_zero_tails<double2>, grid, dim3(256), 0, s, static_cast<double2*>(y), stride, counts_device,
+                                  skip.ptr, skip.stride));
     else
-        k_zero_tails<float2><<<grid, 256, 0, s>>>(static_cast<float2*>(y), stride, counts_device, skip.ptr,
-                                                  skip.stride);
+        RTM_CUDA(launch_dependent(k_zero_tails<float2>, grid, dim3(256), 0, s, static_cast<float2*>(y), stride, counts_device,
+                                  skip.ptr, skip.stride));
     count_launch();
     RTM_CUDA(cudaGetLastError());
     return RTM_OK;

@@ -159,7 +159,6 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_y_fwd(const Gri
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T2* sm = reinterpret_cast<T2*>(smem_raw);
     griddep_wait();
-    griddep_launch_dependents();
     const int c = blockIdx.y, rhs = blockIdx.z;
     if (skipped(a, rhs)) return;
     const PlateDesc<T> pd = plate_of(a, rhs);
@@ -209,7 +208,6 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T2* sm = reinterpret_cast<T2*>(smem_raw);
     griddep_wait();
-    griddep_launch_dependents();
     const int py = blockIdx.y, rhs = blockIdx.z;
     if (skipped(a, rhs)) return;
     const PlateDesc<T> pd = plate_of(a, rhs);
@@ -326,7 +324,6 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
     T2* sst = reinterpret_cast<T2*>(smem_raw + M::lines + M::wrows);
     __shared__ __align__(8) uint64_t bar[2];  // 0: W rows, 1: spectra rows
     griddep_wait();
-    griddep_launch_dependents();
     const int Q = a.Q, per_py = Q / TEAMS, per_rhs = 2 * per_py;
     const int64_t QP = (int64_t)Q * NP;
     const int tid = threadIdx.x;
@@ -465,7 +462,6 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_y_inv(const Gri
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T2* sm = reinterpret_cast<T2*>(smem_raw);
     griddep_wait();
-    griddep_launch_dependents();
     const int c = blockIdx.y, rhs = blockIdx.z;
     if (skipped(a, rhs)) return;
     const PlateDesc<T> pd = plate_of(a, rhs);
@@ -520,7 +516,8 @@ template <typename T, int NQ, int MINB> int launch_y_b(const GridArgs<T>& a, int
     const int rows_max = a.rows[0] > a.rows[1] ? a.rows[0] : a.rows[1];
     const dim3 grid((rows_max + TI - 1) / TI, 2, nrhs);
     if (fwd)
-        k_fast_y_fwd<T, NQ, MINB><<<grid, Fast<T>::threads, smem, s>>>(a, static_cast<const T2*>(x));
+        RTM_CUDA(launch_dependent(k_fast_y_fwd<T, NQ, MINB>, grid, dim3(Fast<T>::threads), smem, s, a,
+                                  static_cast<const T2*>(x)));
     else
         RTM_CUDA(launch_dependent(k_fast_y_inv<T, NQ, MINB>, grid, dim3(Fast<T>::threads), smem, s, a,
                                   static_cast<T2*>(y)));

@@ -12,6 +12,7 @@
 #include "fft.cuh"
 #include "grid.h"
 #include "ops.h"
+#include "pdl.cuh"
 
 namespace rtm {
 
@@ -229,6 +230,7 @@ __device__ __forceinline__ void bj_rows(const BjShape& g, const T2* __restrict__
 template <typename T2>
 __global__ void k_bj_apply(const BjShape g, const T2* __restrict__ x, T2* __restrict__ y, int64_t n, const int* skip,
                            int stride) {
+    griddep_wait();
     const int rhs = blockIdx.y;
     if (skip && skip[(int64_t)rhs * stride]) return;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -240,6 +242,7 @@ __global__ void k_bj_apply(const BjShape g, const T2* __restrict__ x, T2* __rest
 template <typename T2>
 __global__ void k_bj_apply_batch(const BjShape* __restrict__ entries, const T2* __restrict__ x, T2* __restrict__ y,
                                  int64_t stride, const int* skip, int skip_stride) {
+    griddep_wait();
     const int rhs = blockIdx.y;
     if (skip && skip[(int64_t)rhs * skip_stride]) return;
     const BjShape e = entries[rhs];
@@ -253,11 +256,11 @@ int apply_block_jacobi_batch(const BjShape* entries, int count, int max_blocks, 
     const int64_t threads = (int64_t)max_blocks * S;
     const dim3 g((unsigned)((threads + 255) / 256), count);
     if (precision == RTM_FP64)
-        k_bj_apply_batch<double2><<<g, 256, 0, s>>>(entries, static_cast<const double2*>(x), static_cast<double2*>(y),
-                                                    stride, skip.ptr, skip.stride);
+        RTM_CUDA(launch_dependent(k_bj_apply_batch<double2>, g, dim3(256), 0, s, entries, static_cast<const double2*>(x),
+                                  static_cast<double2*>(y), stride, skip.ptr, skip.stride));
     else
-        k_bj_apply_batch<float2><<<g, 256, 0, s>>>(entries, static_cast<const float2*>(x), static_cast<float2*>(y),
-                                                   stride, skip.ptr, skip.stride);
+        RTM_CUDA(launch_dependent(k_bj_apply_batch<float2>, g, dim3(256), 0, s, entries, static_cast<const float2*>(x),
+                                  static_cast<float2*>(y), stride, skip.ptr, skip.stride));
     count_launch();
     RTM_CUDA(cudaGetLastError());
     return RTM_OK;
@@ -270,11 +273,11 @@ struct BlockJacobi : LinearOp {
         const int64_t threads = (int64_t)shape.nbx * shape.nby * shape.S;
         dim3 g((unsigned)((threads + 255) / 256), nrhs);
         if (precision == RTM_FP64)
-            k_bj_apply<double2><<<g, 256, 0, s>>>(shape, static_cast<const double2*>(x), static_cast<double2*>(y), n,
-                                                  skip.ptr, skip.stride);
+            RTM_CUDA(launch_dependent(k_bj_apply<double2>, g, dim3(256), 0, s, shape, static_cast<const double2*>(x),
+                                      static_cast<double2*>(y), n, skip.ptr, skip.stride));
         else
-            k_bj_apply<float2><<<g, 256, 0, s>>>(shape, static_cast<const float2*>(x), static_cast<float2*>(y), n,
-                                                 skip.ptr, skip.stride);
+            RTM_CUDA(launch_dependent(k_bj_apply<float2>, g, dim3(256), 0, s, shape, static_cast<const float2*>(x),
+                                      static_cast<float2*>(y), n, skip.ptr, skip.stride));
         count_launch();
         RTM_CUDA(cudaGetLastError());
         return RTM_OK;
