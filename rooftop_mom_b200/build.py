@@ -16,7 +16,8 @@ OUT = os.path.join(HERE, "librtm.so")
 OBJ = os.path.join(HERE, "_build")
 SOURCES = ["runtime.cpp", "capi.cpp", "server.cpp", "grid.cu", "grid_fast.cu", "assembly.cu", "krylov.cu", "strip_solve.cu", "ops.cu", "excitation.cu", "fixed_scratch.cu", "fault.cu", "tune.cpp", "batch.cu"]
 # sources compiled once for each form, so that their kernels compile side by side: object name -> (source, defines)
-FORMS = {f"grid_reg.{k}": ("grid_reg.cu", [f"-DRTM_REG_FORM={k}"]) for k in range(8)}
+FORMS = {**{f"grid_reg.{k}": ("grid_reg.cu", [f"-DRTM_REG_FORM={k}"]) for k in range(8)},
+         **{f"gen_reg.{k}": ("gen_reg.cu", [f"-DRTM_GEN_FORM={k}"]) for k in range(4)}}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
          "-Wno-deprecated-gpu-targets"]

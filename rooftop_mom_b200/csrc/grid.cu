@@ -20,6 +20,7 @@
 #include <string>
 
 #include "fft.cuh"
+#include "gen.cuh"
 #include "grid.h"
 #include "grid_args.cuh"
 
@@ -559,116 +560,7 @@ int apply_fixed_scratch(const GridApplicator& g, const void* x, void* y, int nrh
 }
 
 // ============================================================================================
-// Spectra builders: 2-D DFTs (P x Q) of generated inputs, in FP64.
-enum SourceKind { kSrcEmbed = 0, kSrcCirculant = 1, kSrcTwoSided = 2, kSrcPart = 3 };
-enum Window { kWinStrang = 0, kWinTChan = 1, kWinRChan = 2, kWinHuckle = 3 };
-constexpr int kMaxItems = 12;
-
-struct GenItem {
-    const double2* g;  // generator, column-major rows x cols (two-sided sources: (2P - 1) x (2Q - 1))
-    int rows, cols;
-    int px, py;        // subband parities; part (m, n) of kSrcPart
-    double2* dst;      // P x Q output (column-major, x fastest)
-};
-
-struct GenArgs {
-    int P, Q;
-    int kind;
-    int Lx, Ly;        // mirror periods of the embedding
-    int nsx, nsy;      // folded copies (2 for split directions)
-    double scale;
-    int window, bw_x, bw_y;
-    int realify;
-    int ti;
-    FftPlan planP, planQ;
-    const double2* twP;
-    const double2* twQ;
-    const double2* modP;
-    const double2* modQ;
-    int nitems;
-    GenItem items[kMaxItems];
-};
-
-__device__ __forceinline__ int mirror_index(int i, int rows, int L) {
-    if (i < rows) return i;
-    const int m = L - i;
-    return (m >= 0 && m < rows) ? m : -1;
-}
-
-__device__ __forceinline__ double window_weight(int w, int o, int n, int bw) {
-    const int ao = o < 0 ? -o : o;
-    switch (w) {
-        case kWinStrang: return (2 * ao < n) ? 1.0 : (2 * ao == n ? 0.5 : 0.0);
-        case kWinTChan: return (double)(n - ao) / (double)n;
-        case kWinRChan: return 1.0;
-        default: return fmax(0.0, 1.0 - (double)ao / (double)bw);
-    }
-}
-
-__device__ double2 gen_value(const GenArgs& a, const GenItem& it, int i, int j) {
-    double re = 0, im = 0;
-    if (a.kind == kSrcEmbed) {
-        for (int ca = 0; ca < a.nsx; ++ca) {
-            const int mx = mirror_index(i + ca * a.P, it.rows, a.Lx);
-            if (mx < 0) continue;
-            const double sa = (it.px && ca) ? -1.0 : 1.0;
-            for (int cb = 0; cb < a.nsy; ++cb) {
-                const int my = mirror_index(j + cb * a.Q, it.cols, a.Ly);
-                if (my < 0) continue;
-                const double sb = (it.py && cb) ? -1.0 : 1.0;
-                const double2 g = it.g[mx + (int64_t)my * it.rows];
-                re += sa * sb * g.x;
-                im += sa * sb * g.y;
-            }
-        }
-        double2 v = make_double2(re * a.scale, im * a.scale);
-        if (it.px) v = cmul(v, a.modP[i]);
-        if (it.py) v = cmul(v, a.modQ[j]);
-        return v;
-    }
-    if (a.kind == kSrcTwoSided || a.kind == kSrcPart) {
-        // A two-sided source, offsets -(P-1)..P-1 by -(Q-1)..Q-1. kSrcTwoSided: the windowed fold onto the
-        // face grid (foldGenerator.m:47-60). kSrcPart: part (m, n) of generatePartSpectra.m:15-49, the
-        // halved sum (m = 0) or difference (m = 1) of the offsets i and i - P, likewise along y, times
-        // exp(i pi i / P) for m = 1 and exp(i pi j / Q) for n = 1.
-        const bool part = a.kind == kSrcPart;
-        for (int ca = 0; ca < 2; ++ca) {
-            if (ca == 1 && i == 0) continue;
-            const int ox = ca ? i - a.P : i;
-            const double wa = part ? ((it.px && ca) ? -0.5 : 0.5) : window_weight(a.window, ox, a.P, a.bw_x);
-            for (int cb = 0; cb < 2; ++cb) {
-                if (cb == 1 && j == 0) continue;
-                const int oy = cb ? j - a.Q : j;
-                const double wb = part ? ((it.py && cb) ? -0.5 : 0.5) : window_weight(a.window, oy, a.Q, a.bw_y);
-                const double2 g = it.g[(ox + a.P - 1) + (int64_t)(oy + a.Q - 1) * it.rows];
-                re += wa * wb * g.x;
-                im += wa * wb * g.y;
-            }
-        }
-        double2 v = make_double2(re, im);
-        if (part && it.px) v = cmulc(v, a.modP[i]);
-        if (part && it.py) v = cmulc(v, a.modQ[j]);
-        return v;
-    }
-    // Circulant fold of the even generator onto the face grid (foldGenerator.m:38-45).
-    for (int ca = 0; ca < 2; ++ca) {
-        if (ca == 1 && i == 0) continue;
-        const int mx = ca ? a.P - i : i;
-        if (mx >= it.rows) continue;
-        const double wa = window_weight(a.window, ca ? i - a.P : i, a.P, a.bw_x);
-        for (int cb = 0; cb < 2; ++cb) {
-            if (cb == 1 && j == 0) continue;
-            const int my = cb ? a.Q - j : j;
-            if (my >= it.cols) continue;
-            const double wb = window_weight(a.window, cb ? j - a.Q : j, a.Q, a.bw_y);
-            const double2 g = it.g[mx + (int64_t)my * it.rows];
-            re += wa * wb * g.x;
-            im += wa * wb * g.y;
-        }
-    }
-    return make_double2(re, im);
-}
-
+// Spectra builders: 2-D DFTs (P x Q) of generated inputs, in FP64 (sources and arguments in gen.cuh).
 __global__ void __launch_bounds__(kMaxThreads, 1) k_gen_y(const GenArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int TI = a.ti, Q = a.Q;
@@ -704,7 +596,20 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_gen_x(const GenArgs a) {
     }
 }
 
-static int run_gen(GenArgs& a, cudaStream_t s) {
+static int reg_gen(bool x, const GenArgs& a, const RegPlan& r, cudaStream_t s) {
+    const bool blue = r.m != r.n;
+    if (r.n1 > 16) return blue ? launch_reg_gen<1, true>(x, a, r, s) : launch_reg_gen<1, false>(x, a, r, s);
+    return blue ? launch_reg_gen<0, true>(x, a, r, s) : launch_reg_gen<0, false>(x, a, r, s);
+}
+
+// The spectra of a.items; rP, rQ: the lengths' register-resident splits (the Stockham kernels serve without).
+static int run_gen(GenArgs& a, const RegPlan& rP, const RegPlan& rQ, cudaStream_t s) {
+    if (a.nitems > 0 && rP.n1 && rQ.n1) {
+        RTM_TRY(reg_gen(false, a, rQ, s));
+        RTM_TRY(reg_gen(true, a, rP, s));
+        RTM_CUDA(cudaGetLastError());
+        return RTM_OK;
+    }
     static DeviceOnce once;
     RTM_TRY(once([]() -> int {
         RTM_CUDA(cudaFuncSetAttribute(k_gen_y, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -899,8 +804,7 @@ int build_product(const DeviceGenerators& g, double size_x, double size_y, int p
         out.mode = kGen3;
         DeviceBuffer raw;
         StreamSyncGuard guard(s);
-        RTM_TRY(raw.alloc((size_t)nsub * 3 * G * sizeof(double2)));
-        RTM_CUDA(cudaMemsetAsync(raw.ptr, 0, raw.bytes, s));
+        RTM_TRY(raw.alloc((size_t)nsub * 3 * G * sizeof(double2)));  // every item is written whole
         for (int sub = 0; sub < nsub; ++sub) {
             for (int k = 0; k < 3; ++k) {
                 GenItem& it = a.items[a.nitems++];
@@ -912,8 +816,9 @@ int build_product(const DeviceGenerators& g, double size_x, double size_y, int p
                 it.dst = raw.as<double2>() + (int64_t)(sub * 3 + k) * G;
             }
         }
-        RTM_TRY(run_gen(a, s));
-        RTM_TRY(convert_spectra(raw, precision, out.spec, s));
+        RTM_TRY(run_gen(a, tP->reg, tQ->reg, s));
+        if (precision == RTM_FP64) out.spec.take(raw);
+        else RTM_TRY(convert_spectra(raw, precision, out.spec, s));
         out.spec_blocks = nsub * 3;
         for (int p = 0; p < out.nsx; ++p) fill_shift(out, out.P, p, true, p);
         for (int p = 0; p < out.nsy; ++p) fill_shift(out, out.Q, p, false, p);
@@ -944,7 +849,7 @@ int build_product(const DeviceGenerators& g, double size_x, double size_y, int p
             it.dst = raw.as<double2>() + (int64_t)(sub * 2 + k) * G;
         }
     }
-    RTM_TRY(run_gen(a, s));
+    RTM_TRY(run_gen(a, tP->reg, tQ->reg, s));
     RTM_TRY(blocks64.alloc((size_t)ns * L * sizeof(double2)));
     const double2* u0 = nullptr;
     const double2* u1 = nullptr;
@@ -1214,7 +1119,7 @@ static int run_two_sided(const TwoSidedSpectra& t, int kind, int window, const d
     it.px = px;
     it.py = py;
     it.dst = dst;
-    return run_gen(a, s);
+    return run_gen(a, t.tP->reg, t.tQ->reg, s);
 }
 
 // Spectrum (P x Q) of the kernel applied to a two-sided source: the windowed fold for strang, tChan,
@@ -1316,7 +1221,7 @@ int build_circulant(const DeviceGenerators& g, double size_x, double size_y, int
             it.px = it.py = 0;
             it.dst = raw.as<double2>() + k * G;
         }
-        RTM_TRY(run_gen(a, s));
+        RTM_TRY(run_gen(a, out.tP->reg, out.tQ->reg, s));
     } else {
         TwoSidedSpectra t{cx, cy, a.window, a.bw_x, a.bw_y, out.tP, out.tQ};
         const int64_t T = (int64_t)(2 * cx - 1) * (2 * cy - 1);
@@ -1380,7 +1285,8 @@ int build_circulant(const DeviceGenerators& g, double size_x, double size_y, int
                                       "or builder.");
     if (out.content == RTM_BOTH) {
         out.mode = kBlock4;
-        RTM_TRY(convert_spectra(inv, precision, out.spec, s));
+        if (precision == RTM_FP64) out.spec.take(inv);
+        else RTM_TRY(convert_spectra(inv, precision, out.spec, s));
         out.spec_blocks = 4;
         out.max_rhs = 0;
         RTM_TRY(out.reserve(1));
