@@ -12,7 +12,7 @@
 // Kernels:
 //   k_far_blocks  - the kernel exp(-ikR)/R on the far lattice: block (m, n) holds the order^2
 //                   points x = a (p - m), y = b (p - n); each block's four quadrant sums of the 7
-//                   moment weights (28 complex numbers) are written out. FP64 sincos/sqrt/div bound.
+//                   moment weights (28 complex numbers) are written out.
 //   k_near        - one CTA per near offset: 7 weighted sums over the near rule, the remainder of
 //                   the singularity extraction on the touching offsets plus their closed form.
 //   k_terms       - per offset: the moments (near, or four quadrant sums of the far blocks) and
@@ -30,69 +30,134 @@ namespace rtm {
 static constexpr double kZ0 = 376.730313668;  // Constants.m:11
 static constexpr double kPi = 3.141592653589793238462643383279502884;
 
-constexpr int kBlocksPerCta = 32;
-constexpr int kPointChunk = 64;
+// The moment weights are products of one-dimensional ones (generateReducedRule.m:33): of the nodes of an axis
+// ([4] columns W00, W10, W01, W11), M00, M10, M01, M11 are W00(eta) W..(nu) and N10, N01, N11 are W..(eta) W00(nu).
+__device__ __forceinline__ double moment_weight(int m, const double* wx, int sx, const double* wy, int sy) {
+    return m < 4 ? wy[0] * wx[m * sx] : wy[(m - 3) * sy] * wx[0];
+}
 
 struct FarArgs {
     int cx, cy;        // faces; blocks are 0..cx x 0..cy
     int order;
+    int square;        // square faces: block (n, m) mirrors block (m, n)
+    int staged;        // the rule in shared memory
+    int64_t nblocks;   // blocks evaluated
     double a, b, k;
     const double* points;   // order far points p in (0, 1)
-    const double* weights;  // [4 quadrants][7][order^2], point index px + order * py
+    const double* weights;  // [2 halves][4][order], of one axis
     double2* sums;          // [28][(cx+1)(cy+1)], block index m + (cx+1) n
 };
 
-__global__ void __launch_bounds__(128) k_far_blocks(const FarArgs f) {
-    __shared__ double2 K[kPointChunk][kBlocksPerCta];
-    __shared__ double W[4][7][kPointChunk];
-    const int64_t nblocks = (int64_t)(f.cx + 1) * (f.cy + 1);
-    const int64_t first = (int64_t)blockIdx.x * kBlocksPerCta;
-    const int tb = threadIdx.x % kBlocksPerCta;  // block within the CTA (lane)
-    const int q = threadIdx.x / kBlocksPerCta;   // quadrant (warp)
-    const int npts = f.order * f.order;
-    double re[7], im[7];
+// The evaluated blocks in order: all of them, or with square faces those of m >= n and the rows n > cx, whose mirror
+// images lie outside.
+__device__ __forceinline__ void far_block(const FarArgs& f, int64_t t, int& m, int& n) {
+    const int64_t W = f.cx + 1;
+    if (!f.square) {
+        n = (int)(t / W);
+        m = (int)(t - n * W);
+        return;
+    }
+    const int64_t last = min(f.cx, f.cy) + (int64_t)1;          // triangular rows: row n holds W - n blocks
+    const int64_t tri = last * W - last * (last - 1) / 2;
+    if (t >= tri) {
+        n = (int)(last + (t - tri) / W);
+        m = (int)((t - tri) % W);
+        return;
+    }
+    // the largest n with n W - n (n - 1) / 2 <= t, from the quadratic's root, corrected for its rounding
+    const double h = W + 0.5;
+    int64_t q = (int64_t)(h - sqrt(fmax(0.0, h * h - 2.0 * (double)t)));
+    q = max((int64_t)0, min(q, last - 1));
+    while (q > 0 && q * W - q * (q - 1) / 2 > t) --q;
+    while (q + 1 < last && (q + 1) * W - (q + 1) * q / 2 <= t) ++q;
+    n = (int)q;
+    m = (int)(t - (q * W - q * (q - 1) / 2) + q);
+}
+
+// A thread per (block, row of points py) evaluates the kernel at its row's points and sums them with the weights along
+// x (2 halves x 4 columns) in registers; a thread per (block, quadrant) then sums those along y. Against a thread per
+// (block, quadrant) over all points and weights that is 1472 multiply-adds a block instead of 3584, at order 8, and
+// no kernel value goes through shared memory; square faces evaluate half the blocks. Bound: the FP64 square root,
+// sine, cosine and reciprocal of 64 points a block. 256 x 256 blocks: 66 us before, 1024 x 1024: 924 us.
+constexpr int kFarThreads = 256, kFarRows = 32;  // rows of points a pass takes at most
+
+__global__ void __launch_bounds__(kFarThreads) k_far_blocks(const FarArgs f, int py_threads) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int o = f.order, nb = kFarThreads / py_threads;  // blocks of the CTA
+    double2* A = reinterpret_cast<double2*>(smem_raw);      // [py_threads][2 x 4][nb]
+    const double* w = f.weights;  // [2][4][order], in shared memory where they fit
+    const double* pts = f.points;
+    if (f.staged) {
+        double* sw = reinterpret_cast<double*>(A + (size_t)py_threads * 8 * nb);
+        double* sp = sw + 8 * o;
+        for (int t = threadIdx.x; t < 8 * o; t += kFarThreads) sw[t] = f.weights[t];
+        for (int t = threadIdx.x; t < o; t += kFarThreads) sp[t] = f.points[t];
+        w = sw;
+        pts = sp;
+    }
+    const int64_t first = (int64_t)blockIdx.x * nb, W = f.cx + 1, total = W * (f.cy + 1);
+    const int bl = threadIdx.x % nb, row = threadIdx.x / nb;  // block of the CTA; row of points
+    const bool in = first + bl < f.nblocks;
+    int m = 0, n = 0;
+    if (in) far_block(f, first + bl, m, n);
+    double2 M[7];
 #pragma unroll
-    for (int m = 0; m < 7; ++m) re[m] = im[m] = 0.0;
-    for (int p0 = 0; p0 < npts; p0 += kPointChunk) {
-        const int np = min(kPointChunk, npts - p0);
-        for (int t = threadIdx.x; t < kPointChunk * kBlocksPerCta; t += blockDim.x) {
-            const int bl = t % kBlocksPerCta, pt = t / kBlocksPerCta;
-            const int64_t blk = first + bl;
-            double2 v = make_double2(0.0, 0.0);
-            if (pt < np && blk < nblocks) {
-                const int m = (int)(blk % (f.cx + 1)), n = (int)(blk / (f.cx + 1));
-                const int gp = p0 + pt;
-                const int px = gp % f.order, py = gp / f.order;
-                const double x = f.a * (f.points[px] - m);
-                const double y = f.b * (f.points[py] - n);
-                const double R = sqrt(x * x + y * y);
+    for (int e = 0; e < 7; ++e) M[e] = make_double2(0, 0);
+    const int hx = row & 1, hy = (row >> 1) & 1;  // this thread's quadrant in the second part (rows 0 to 3)
+    __syncthreads();
+    for (int p0 = 0; p0 < o; p0 += py_threads) {
+        const int py = p0 + row;
+        double2 S[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) S[e] = make_double2(0, 0);
+        if (in && py < o) {
+            const double y = f.b * (pts[py] - n), y2 = y * y;
+            for (int px = 0; px < o; ++px) {
+                const double x = f.a * (pts[px] - m);
+                const double R = sqrt(x * x + y2);
                 double s, c;
                 sincos(f.k * R, &s, &c);
                 const double inv = 1.0 / R;
-                v = make_double2(c * inv, -s * inv);
-            }
-            K[pt][bl] = v;
-        }
-        for (int t = threadIdx.x; t < 4 * 7 * kPointChunk; t += blockDim.x) {
-            const int pt = t % kPointChunk, r = t / kPointChunk;
-            (&W[0][0][0])[t] = pt < np ? f.weights[(int64_t)r * npts + p0 + pt] : 0.0;
-        }
-        __syncthreads();
-        for (int pt = 0; pt < np; ++pt) {
-            const double2 kv = K[pt][tb];
+                const double kr = c * inv, ki = -s * inv;
 #pragma unroll
-            for (int m = 0; m < 7; ++m) {
-                const double w = W[q][m][pt];
-                re[m] = fma(w, kv.x, re[m]);
-                im[m] = fma(w, kv.y, im[m]);
+                for (int e = 0; e < 8; ++e) {
+                    S[e].x = fma(w[e * o + px], kr, S[e].x);
+                    S[e].y = fma(w[e * o + px], ki, S[e].y);
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) A[(row * 8 + e) * nb + bl] = S[e];
+        __syncthreads();
+        if (row < 4) {
+            const int rows = min(py_threads, o - p0);
+            for (int q = rows - 1; q >= 0; --q) {
+                const double* wy = w + hy * 4 * o + p0 + q;
+                double2 a[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) a[e] = A[(q * 8 + hx * 4 + e) * nb + bl];
+#pragma unroll
+                for (int e = 0; e < 7; ++e) {
+                    const double ww = e < 4 ? wy[0] : wy[(e - 3) * o];
+                    const double2 v = e < 4 ? a[e] : a[0];
+                    M[e].x = fma(ww, v.x, M[e].x);
+                    M[e].y = fma(ww, v.y, M[e].y);
+                }
             }
         }
         __syncthreads();
     }
-    const int64_t blk = first + tb;
-    if (blk < nblocks) {
+    if (row >= 4 || !in) return;
+    const int64_t at = m + W * n;
+    const int q = hx + 2 * hy;
 #pragma unroll
-        for (int m = 0; m < 7; ++m) f.sums[(int64_t)(q * 7 + m) * nblocks + blk] = make_double2(re[m], im[m]);
+    for (int e = 0; e < 7; ++e) f.sums[(int64_t)(q * 7 + e) * total + at] = M[e];
+    if (f.square && m != n && n <= f.cx && m <= f.cy) {
+        // x and y exchanged: quadrant (hy, hx) of block (n, m), the M.. and the N.. (M00 is its own image)
+        const int64_t mirror = n + W * m;
+        const int qm = hy + 2 * hx;
+#pragma unroll
+        for (int e = 0; e < 7; ++e) f.sums[(int64_t)(qm * 7 + (e == 0 ? 0 : e < 4 ? e + 3 : e - 3)) * total + mirror] = M[e];
     }
 }
 
@@ -102,7 +167,8 @@ struct NearArgs {
     double a, b, k;
     const double* nodes_x;
     const double* nodes_y;
-    const double* weights;    // [7][px_count * py_count], nu fastest
+    const double* weights_x;  // [px_count][4], [py_count][4]
+    const double* weights_y;
     const double* extracted;  // [7][4] closed-form moments at (0,0), (1,0), (0,1), (1,1)
     int count_x, count_y;
     double2* moments;         // [near_x * near_y][7], offset dX + near_x dY
@@ -141,7 +207,7 @@ __global__ void __launch_bounds__(256) k_near(const NearArgs f) {
         }
 #pragma unroll
         for (int m = 0; m < 7; ++m) {
-            const double w = f.weights[(int64_t)m * npts + p];
+            const double w = moment_weight(m, f.weights_x + 4 * ix, 1, f.weights_y + 4 * iy, 1);
             re[m] = fma(w, kv.x, re[m]);
             im[m] = fma(w, kv.y, im[m]);
         }
@@ -290,34 +356,11 @@ static void reduced_axis(int order, int parts, std::vector<double>& nodes, std::
             }
 }
 
-// 7 x (Px*Py) weights, nu fastest: rows M00, M10, M01, M11 = W00(eta) W..(nu), rows N10, N01, N11
-// = W..(eta) W00(nu) (generateReducedRule.m:33).
-static void reduced_rule(int order, int parts_x, int parts_y, std::vector<double>& nx, std::vector<double>& ny,
-                         std::vector<double>& weights) {
-    std::vector<double> wx, wy;
-    reduced_axis(order, parts_x, nx, wx);
-    reduced_axis(order, parts_y, ny, wy);
-    const int Px = (int)nx.size(), Py = (int)ny.size();
-    weights.assign((size_t)7 * Px * Py, 0.0);
-    for (int iy = 0; iy < Py; ++iy)
-        for (int ix = 0; ix < Px; ++ix) {
-            const size_t col = (size_t)iy * Px + ix;
-            for (int r = 0; r < 4; ++r) weights[(size_t)r * Px * Py + col] = wy[(size_t)iy * 4] * wx[(size_t)ix * 4 + r];
-            for (int r = 1; r < 4; ++r) weights[(size_t)(3 + r) * Px * Py + col] = wy[(size_t)iy * 4 + r] * wx[(size_t)ix * 4];
-        }
-}
-
 static int count_near(int count, double size, double longest) {
     int n = 0;
     for (int d = 0; d < count; ++d)
         if (std::max(d - 1, 0) * size < 3 * longest) ++n;
     return n;
-}
-
-template <typename V> static int upload(DeviceBuffer& buf, const std::vector<V>& v, cudaStream_t s) {
-    RTM_TRY(buf.alloc(v.size() * sizeof(V)));
-    RTM_CUDA(cudaMemcpyAsync(buf.ptr, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, s));
-    return RTM_OK;
 }
 
 int assemble_generators(int cx, int cy, double a, double b, double k, int near_order, int far_order,
@@ -344,21 +387,37 @@ int assemble_generators(int cx, int cy, double a, double b, double k, int near_o
     const double shortest = std::min(a, b);
     const int parts_x = (int)std::floor(a / shortest + 0.5), parts_y = (int)std::floor(b / shortest + 0.5);
 
-    // Near pass.
-    std::vector<double> nnx, nny, nw;
-    reduced_rule(near_order, parts_x, parts_y, nnx, nny, nw);
+    // The rules of both passes and the closed forms, uploaded together.
+    std::vector<double> host;
+    auto put = [&](const std::vector<double>& v) {
+        const size_t at = host.size();
+        host.insert(host.end(), v.begin(), v.end());
+        return at;
+    };
+    std::vector<double> nnx, nny, nwx, nwy, fnx, fw;
+    reduced_axis(near_order, parts_x, nnx, nwx);
+    reduced_axis(near_order, parts_y, nny, nwy);
+    reduced_axis(far_order, 1, fnx, fw);
     double ext[7][4];
     extracted_moments(a, b, k, ext);
-    std::vector<double> extv(28);
-    for (int r = 0; r < 7; ++r)
-        for (int c = 0; c < 4; ++c) extv[r * 4 + c] = ext[r][c];
-    DeviceBuffer d_nx, d_ny, d_nw, d_ext, d_near, d_pts, d_qw, d_sums, d_terms;
+    const int o = far_order;
+    std::vector<double> axis((size_t)8 * o);  // [half][column][point] of the far rule, whose axes are alike
+    for (int h = 0; h < 2; ++h)
+        for (int c = 0; c < 4; ++c)
+            for (int i = 0; i < o; ++i) axis[(size_t)(h * 4 + c) * o + i] = fw[(size_t)(h * o + i) * 4 + c];
+    const size_t at_nx = put(nnx), at_ny = put(nny), at_wx = put(nwx), at_wy = put(nwy),
+                 at_ext = put(std::vector<double>(&ext[0][0], &ext[0][0] + 28)),
+                 at_pts = put(std::vector<double>(fnx.begin() + o, fnx.end())), at_axis = put(axis);
+    const int64_t nblocks = (int64_t)(cx + 1) * (cy + 1);
+    DeviceBuffer d_host, d_near, d_sums, d_terms;
     StreamSyncGuard guard(s);
-    RTM_TRY(upload(d_nx, nnx, s));
-    RTM_TRY(upload(d_ny, nny, s));
-    RTM_TRY(upload(d_nw, nw, s));
-    RTM_TRY(upload(d_ext, extv, s));
+    RTM_TRY(d_host.alloc(host.size() * sizeof(double)));
     RTM_TRY(d_near.alloc((size_t)near_x * near_y * 7 * sizeof(double2)));
+    RTM_TRY(d_sums.alloc((size_t)28 * nblocks * sizeof(double2)));
+    RTM_CUDA(cudaMemcpyAsync(d_host.ptr, host.data(), d_host.bytes, cudaMemcpyHostToDevice, s));
+    const double* dev = d_host.as<double>();
+
+    // Near pass.
     NearArgs na{};
     na.near_x = near_x;
     na.near_y = near_y;
@@ -367,10 +426,11 @@ int assemble_generators(int cx, int cy, double a, double b, double k, int near_o
     na.a = a;
     na.b = b;
     na.k = k;
-    na.nodes_x = d_nx.as<double>();
-    na.nodes_y = d_ny.as<double>();
-    na.weights = d_nw.as<double>();
-    na.extracted = d_ext.as<double>();
+    na.nodes_x = dev + at_nx;
+    na.nodes_y = dev + at_ny;
+    na.weights_x = dev + at_wx;
+    na.weights_y = dev + at_wy;
+    na.extracted = dev + at_ext;
     na.count_x = cx;
     na.count_y = cy;
     na.moments = d_near.as<double2>();
@@ -379,36 +439,30 @@ int assemble_generators(int cx, int cy, double a, double b, double k, int near_o
     RTM_CUDA(cudaGetLastError());
 
     // Far lattice (quadrant weights of the far rule, one part per direction).
-    std::vector<double> fnx, fny, fw;
-    reduced_rule(far_order, 1, 1, fnx, fny, fw);
-    const int o = far_order, P2 = 2 * o;
-    std::vector<double> points(fnx.begin() + o, fnx.end());
-    std::vector<double> qw((size_t)4 * 7 * o * o);
-    for (int hy = 0; hy < 2; ++hy)
-        for (int hx = 0; hx < 2; ++hx) {
-            const int q = hx + 2 * hy;
-            for (int m = 0; m < 7; ++m)
-                for (int py = 0; py < o; ++py)
-                    for (int px = 0; px < o; ++px) {
-                        const size_t col = (size_t)(hy * o + py) * P2 + (hx * o + px);
-                        qw[((size_t)q * 7 + m) * o * o + px + (size_t)o * py] = fw[(size_t)m * P2 * P2 + col];
-                    }
-        }
-    RTM_TRY(upload(d_pts, points, s));
-    RTM_TRY(upload(d_qw, qw, s));
-    const int64_t nblocks = (int64_t)(cx + 1) * (cy + 1);
-    RTM_TRY(d_sums.alloc((size_t)28 * nblocks * sizeof(double2)));
     FarArgs fa{};
     fa.cx = cx;
     fa.cy = cy;
     fa.order = o;
+    fa.square = a == b;
+    fa.nblocks = nblocks;
+    if (fa.square) {
+        const int64_t last = std::min(cx, cy) + (int64_t)1;
+        fa.nblocks -= last * (last - 1) / 2;  // the blocks that mirror another one
+    }
     fa.a = a;
     fa.b = b;
     fa.k = k;
-    fa.points = d_pts.as<double>();
-    fa.weights = d_qw.as<double>();
+    fa.points = dev + at_pts;
+    fa.weights = dev + at_axis;
     fa.sums = d_sums.as<double2>();
-    k_far_blocks<<<(unsigned)((nblocks + kBlocksPerCta - 1) / kBlocksPerCta), 128, 0, s>>>(fa);
+    // a power of two of point rows, at least the four a block's quadrants need
+    int py_threads = 4;
+    while (py_threads < std::min(o, kFarRows)) py_threads *= 2;
+    const int64_t per_cta = kFarThreads / py_threads;
+    const size_t values = (size_t)kFarThreads * 8 * sizeof(double2), rule = (size_t)9 * o * sizeof(double);
+    fa.staged = values + rule <= 48 * 1024;  // orders up to 227; longer rules are read through the caches
+    const size_t far_smem = values + (fa.staged ? rule : 0);
+    k_far_blocks<<<(unsigned)((fa.nblocks + per_cta - 1) / per_cta), kFarThreads, far_smem, s>>>(fa, py_threads);
     count_launch();
     RTM_CUDA(cudaGetLastError());
 

@@ -191,3 +191,21 @@ def test_arnoldi_steps_whose_basis_spans_the_solution():
     res = R.Solver("gmres", tolerance=1e-12, maxIterationCount=40, restart=20).solve(R.DenseOperator(A), b)
     assert res.converged() and res.iterationCount() == 3
     assert rel(A @ res.solution(), b) < 1e-12
+
+
+@pytest.mark.parametrize("grid", [(1, 2), (2, 1), (2, 2), (3, 7), (7, 3), (31, 33), (40, 40), (64, 5), (5, 64), (90, 1)])
+@pytest.mark.parametrize("sizes,orders", [((0.05, 0.05), (16, 8)), ((0.05, 0.05), (4, 1)), ((0.07, 0.05), (5, 3)),
+                                          ((0.05, 0.05), (6, 33)), ((0.02, 0.05), (4, 5))])
+def test_assembled_generators(grid, sizes, orders):
+    """Square faces (half the far blocks evaluated, the others mirrored) and others, grids wider and taller than the
+    triangle of mirrored blocks, and rules from one point to more rows than a pass takes: the oracle's generators to
+    1e-12 in norm."""
+    import rooftop_mom_b200 as R
+    from oracle import assembly as A
+
+    prob = R.Problem(R.Mesh(*grid, *sizes), K, quadratureOrder=orders)
+    got = prob.generators().arrays()
+    want = A.generate(*grid, *sizes, K, orders)
+    for g, w in zip(got, (want.magnetic_xx, want.magnetic_yy, want.electric)):
+        if w is not None and w.size:
+            assert rel(g, w) < 1e-12
