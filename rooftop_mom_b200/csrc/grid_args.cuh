@@ -29,6 +29,10 @@ template <typename T> struct GridArgs {
     FftPlan planP, planQ;
     const T2* twP;
     const T2* twQ;
+    const T2* taP;  // the twiddles of power-of-two lengths' splits (FftTables)
+    const T2* tbP;
+    const T2* taQ;
+    const T2* tbQ;
     const T2* modP;
     const T2* modQ;
     T2* work;

@@ -49,8 +49,7 @@ __host__ __device__ constexpr double root32_im(int k) { return k <= 8 ? -cos_pi1
 
 // In-register DFT of R points, natural order in and out. R = 32 splits by decimation in frequency
 // into two 16-point transforms with the roots w_32^k (constants, no table reads).
-template <int R, bool INV, typename T2>
-__device__ __forceinline__ void dft_reg(T2 (&v)[R], const T2* __restrict__ tw, int n) {
+template <int R, bool INV, typename T2> __device__ __forceinline__ void dft_reg(T2 (&v)[R]) {
     if constexpr (R == 4) {
         dft4<INV>(v[0], v[1], v[2], v[3]);
     } else if constexpr (R == 8) {
@@ -92,30 +91,29 @@ template <typename T2> struct LineBuf {
 };
 
 // Forward transform of the group's line, steps before the exchange: v[m1] = x[R2 m1 + t] in,
-// written to buf(k1, t).
+// written to buf(k1, t). ta, tb (inv_first): the twiddles in the two orders of FftTables (n1 = R1, n2 = R2).
 template <int N, typename T2>
-__device__ __forceinline__ void fwd_first(T2 (&v)[Shape<N>::R1], int t, const T2* __restrict__ tw,
+__device__ __forceinline__ void fwd_first(T2 (&v)[Shape<N>::R1], int t, const T2* __restrict__ ta,
                                           const LineBuf<T2>& buf) {
     constexpr int R1 = Shape<N>::R1;
-    dft_reg<R1, false>(v, tw, N);
+    dft_reg<R1, false>(v);
 #pragma unroll
     for (int k1 = 0; k1 < R1; ++k1) {
-        const T2 w = k1 ? cmul(v[k1], __ldg(&tw[t * k1])) : v[k1];
+        const T2 w = k1 ? cmul(v[k1], __ldg(&ta[k1 * Shape<N>::R2 + t])) : v[k1];
         buf.at(k1, t) = w;
     }
 }
 
 // After the exchange: v[s R2 + k2] = X[(t + R2 s) + R1 k2].
 template <int N, typename T2>
-__device__ __forceinline__ void fwd_second(T2 (&v)[Shape<N>::R1], int t, const T2* __restrict__ tw,
-                                           const LineBuf<T2>& buf) {
+__device__ __forceinline__ void fwd_second(T2 (&v)[Shape<N>::R1], int t, const LineBuf<T2>& buf) {
     constexpr int R1 = Shape<N>::R1, R2 = Shape<N>::R2, S = R1 / R2;
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         T2 u[R2];
 #pragma unroll
         for (int m2 = 0; m2 < R2; ++m2) u[m2] = buf.at(t + R2 * s, m2);
-        dft_reg<R2, false>(u, tw, N);
+        dft_reg<R2, false>(u);
 #pragma unroll
         for (int k2 = 0; k2 < R2; ++k2) v[s * R2 + k2] = u[k2];
     }
@@ -123,7 +121,7 @@ __device__ __forceinline__ void fwd_second(T2 (&v)[Shape<N>::R1], int t, const T
 
 // Inverse from the transformed layout, steps before the exchange: written to buf(k1, m2) twiddled.
 template <int N, typename T2>
-__device__ __forceinline__ void inv_first(T2 (&v)[Shape<N>::R1], int t, const T2* __restrict__ tw,
+__device__ __forceinline__ void inv_first(T2 (&v)[Shape<N>::R1], int t, const T2* __restrict__ tb,
                                           const LineBuf<T2>& buf) {
     constexpr int R1 = Shape<N>::R1, R2 = Shape<N>::R2, S = R1 / R2;
 #pragma unroll
@@ -131,21 +129,20 @@ __device__ __forceinline__ void inv_first(T2 (&v)[Shape<N>::R1], int t, const T2
         T2 u[R2];
 #pragma unroll
         for (int k2 = 0; k2 < R2; ++k2) u[k2] = v[s * R2 + k2];
-        dft_reg<R2, true>(u, tw, N);
+        dft_reg<R2, true>(u);
         const int k1 = t + R2 * s;
 #pragma unroll
-        for (int m2 = 0; m2 < R2; ++m2) buf.at(k1, m2) = (m2 && k1) ? cmulc(u[m2], __ldg(&tw[m2 * k1])) : u[m2];
+        for (int m2 = 0; m2 < R2; ++m2) buf.at(k1, m2) = m2 ? cmulc(u[m2], __ldg(&tb[m2 * R1 + k1])) : u[m2];
     }
 }
 
 // After the exchange: v[m1] = N x[R2 m1 + t] (unnormalised).
 template <int N, typename T2>
-__device__ __forceinline__ void inv_second(T2 (&v)[Shape<N>::R1], int t, const T2* __restrict__ tw,
-                                           const LineBuf<T2>& buf) {
+__device__ __forceinline__ void inv_second(T2 (&v)[Shape<N>::R1], int t, const LineBuf<T2>& buf) {
     constexpr int R1 = Shape<N>::R1;
 #pragma unroll
     for (int k1 = 0; k1 < R1; ++k1) v[k1] = buf.at(k1, t);
-    dft_reg<R1, true>(v, tw, N);
+    dft_reg<R1, true>(v);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -178,9 +175,9 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_y_fwd(const Gri
         if (py) e = cmul(e, __ldg(&a.modQ[j]));
         v[m1] = e;
     }
-    fwd_first<NQ>(v, t, a.twQ, buf);
+    fwd_first<NQ>(v, t, a.taQ, buf);
     __syncthreads();
-    fwd_second<NQ>(v, t, a.twQ, buf);
+    fwd_second<NQ>(v, t, buf);
     if (!on) return;
     T2* dst = a.work + (int64_t)rhs * a.work_rhs + (int64_t)(py * a.ncomp + c) * NQ * a.P + i;
 #pragma unroll
@@ -230,9 +227,9 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
         if (px) e = cmul(e, __ldg(&a.modP[i]));
         v[m1] = e;
     }
-    fwd_first<NP>(v, t, a.twP, buf);
+    fwd_first<NP>(v, t, a.taP, buf);
     __syncthreads();
-    fwd_second<NP>(v, t, a.twP, buf);
+    fwd_second<NP>(v, t, buf);
     __syncthreads();  // the buffers are read; they now carry the spectra values to the partner
 #pragma unroll
     for (int r = 0; r < R1; ++r) own[r * R2 + t] = v[r];
@@ -267,9 +264,9 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
             }
     }
     __syncthreads();  // the partner values are read
-    inv_first<NP>(v, t, a.twP, buf);
+    inv_first<NP>(v, t, a.tbP, buf);
     __syncthreads();
-    inv_second<NP>(v, t, a.twP, buf);
+    inv_second<NP>(v, t, buf);
     __syncthreads();
     if (px) {
 #pragma unroll
@@ -389,9 +386,9 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
         }
         __syncthreads();  // the W rows are in registers: the next iteration's may come in
         if (tid == 0 && nxt < iters) issue(nxt, true, false);
-        fwd_first<NP>(v, t, a.twP, buf);
+        fwd_first<NP>(v, t, a.taP, buf);
         __syncthreads();
-        fwd_second<NP>(v, t, a.twP, buf);
+        fwd_second<NP>(v, t, buf);
         __syncthreads();  // the buffers are read; they now carry the spectra values to the partner
 #pragma unroll
         for (int q = 0; q < R1; ++q) own[q * R2 + t] = v[q];
@@ -427,9 +424,9 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
         }
         __syncthreads();  // the spectra and the partner values are read
         if (tid == 0 && nxt < iters) issue(nxt, false, true);
-        inv_first<NP>(v, t, a.twP, buf);
+        inv_first<NP>(v, t, a.tbP, buf);
         __syncthreads();
-        inv_second<NP>(v, t, a.twP, buf);
+        inv_second<NP>(v, t, buf);
         __syncthreads();
         if (px) {
 #pragma unroll
@@ -479,9 +476,9 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_y_inv(const Gri
 #pragma unroll
         for (int k2 = 0; k2 < R2; ++k2)
             v[s * R2 + k2] = on ? src[(int64_t)((t + R2 * s) + R1 * k2) * a.P] : czero<T2>();
-    inv_first<NQ>(v, t, a.twQ, buf);
+    inv_first<NQ>(v, t, a.tbQ, buf);
     __syncthreads();
-    inv_second<NQ>(v, t, a.twQ, buf);
+    inv_second<NQ>(v, t, buf);
     __syncthreads();
     if (py) {
 #pragma unroll

@@ -141,6 +141,14 @@ struct RegPlan {
 struct FftTables {
     FftPlan plan;
     RegPlan reg;
+    // Powers of two from 32 to kRegMax, for grid_fast.cu: the twiddles w^(t k1) of the split n = n1 n2 (t < n2, k1 < n1)
+    // as its two steps read them, consecutive threads on consecutive entries: at k1 n2 + t, and at t n1 + k1. (Gathered
+    // from the roots at t k1, a load touched up to 16 lines: FP32 1024 x 1024 product 140 us, 129 with these. The lines
+    // of grid_reg.cu, whose y passes share a t between 8 threads, gained nothing and lost cache.)
+    const double2* ta64;
+    const double2* tb64;
+    const float2* ta32;
+    const float2* tb32;
     const double2* tw64;   // n entries
     const float2* tw32;
     const double2* mod64;  // exp(-i pi d / n), d < n (the odd-subband modulation)
