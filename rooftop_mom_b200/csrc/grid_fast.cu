@@ -192,6 +192,15 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_y_fwd(const Gri
 // 25 MB instead of 100).
 __device__ __forceinline__ int even_freq(int m, int p, int n) { return min(m, n - m - p); }
 
+// The R2 <= 32 threads of an x line are lanes of one warp, so its exchanges need no CTA barrier. FP32 takes that (1024 x
+// 1024 product 128 -> 125 us, eight 512 x 512 ones 199 -> 190); FP64, whose CTAs hold four warps with up to 255
+// registers, keeps the barriers: its warps then share the twiddle and spectra lines (512 x 512 product 51 us without
+// them, 47 with).
+template <typename T> __device__ __forceinline__ void line_sync() {
+    if constexpr (sizeof(T) == 8) __syncthreads();
+    else __syncwarp();
+}
+
 // x-mix, direct form (one CTA per TEAMS y frequencies; inputs loaded straight into registers, the spectra
 // read in the mix): teams of four groups (component c, x subband px) per y frequency j of subband py. Thread
 // index t + R2 (team * 4 + 2 px + c). Forward transform along x of W mod_x^px, the 2x2 block mix
@@ -215,8 +224,6 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
     const int Q = a.Q;
     const int64_t QP = (int64_t)Q * NP;
     const LineBuf<T2> buf{sm + gid * LB, R2 + 1, 1};
-    T2* own = sm + gid * LB;
-    const T2* partner = sm + (gid ^ 1) * LB;
     const int rows = pd.rows[c];
     T2* row = a.work + (int64_t)rhs * a.work_rhs + (int64_t)(py * a.ncomp + c) * QP + (int64_t)(on ? j : 0) * NP;
     T2 v[R1];
@@ -228,17 +235,25 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
         v[m1] = e;
     }
     fwd_first<NP>(v, t, a.taP, buf);
-    __syncthreads();
+    line_sync<T>();
     fwd_second<NP>(v, t, buf);
-    __syncthreads();  // the buffers are read; they now carry the spectra values to the partner
+    // The partner's values come by warp shuffles where both lines share a warp (FP32; an FP64 value takes four: the
+    // 256 x 256 product 17.2 us with them, 16.1 without), else through the buffers.
+    constexpr bool kShuffle = R2 <= 16 && sizeof(T) == 4;
+    T2* own = sm + gid * LB;
+    const T2* partner = sm + (gid ^ 1) * LB;
+    if constexpr (!kShuffle) {
+        line_sync<T>();  // the line's buffer is read; it now carries the spectra values to the partner
 #pragma unroll
-    for (int r = 0; r < R1; ++r) own[r * R2 + t] = v[r];
-    __syncthreads();
-    if (on) {
+        for (int r = 0; r < R1; ++r) own[r * R2 + t] = v[r];
+        __syncthreads();
+    }
+    if (kShuffle || on) {
         const int sub = px + 2 * py;
-        const T2* spec = pd.spec + (int64_t)(sub * 3) * QP + (int64_t)even_freq(j, py, Q) * NP;
+        const int jc = on ? j : 0;
+        const T2* spec = pd.spec + (int64_t)(sub * 3) * QP + (int64_t)even_freq(jc, py, Q) * NP;
         const T2* ux = px ? a.ux1 : a.ux0;
-        const T2 vv = __ldg(&(py ? a.vy1 : a.vy0)[j]);
+        const T2 vv = __ldg(&(py ? a.vy1 : a.vy0)[jc]);
         const T cv = (vv.x * vv.x + vv.y * vv.y) * pd.inv_b2;
 #pragma unroll
         for (int s = 0; s < S; ++s)
@@ -256,29 +271,36 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
                 qc.y = -qc.y * pd.inv_ab;
                 const T2 coupling = c ? cconj(qc) : qc;
                 const T cself = c ? cv : cu;
-                const T2 me = v[s * R2 + k2], other = partner[(s * R2 + k2) * R2 + t];
+                const T2 me = v[s * R2 + k2];
+                T2 other;
+                if constexpr (kShuffle) {
+                    other.x = __shfl_xor_sync(0xffffffffu, me.x, R2);
+                    other.y = __shfl_xor_sync(0xffffffffu, me.y, R2);
+                } else {
+                    other = partner[(s * R2 + k2) * R2 + t];
+                }
                 // M me - cself E me + coupling E other = M me + E (coupling other - cself me)
                 const T2 cp = cmul(coupling, other);
                 const T2 d = make_vec2<T2>(cp.x - cself * me.x, cp.y - cself * me.y);
                 v[s * R2 + k2] = cadd(cmul(M, me), cmul(E, d));
             }
     }
-    __syncthreads();  // the partner values are read
+    if constexpr (!kShuffle) __syncthreads();  // the partner values are read
     inv_first<NP>(v, t, a.tbP, buf);
-    __syncthreads();
+    line_sync<T>();
     inv_second<NP>(v, t, buf);
-    __syncthreads();
     if (px) {
+        // in the thread's own column of the buffer, which no other one has read
 #pragma unroll
-        for (int m1 = 0; m1 < R1; ++m1) own[m1 * R2 + t] = cmulc(v[m1], __ldg(&a.modP[R2 * m1 + t]));
+        for (int m1 = 0; m1 < R1; ++m1) buf.at(m1, t) = cmulc(v[m1], __ldg(&a.modP[R2 * m1 + t]));
     }
     __syncthreads();
     if (px || !on) return;
-    const T2* odd = sm + (gid + 2) * LB;
+    const LineBuf<T2> odd{sm + (gid + 2) * LB, R2 + 1, 1};
 #pragma unroll
     for (int m1 = 0; m1 < R1; ++m1) {
         const int i = R2 * m1 + t;
-        if (i < rows) row[i] = cscale(cadd(v[m1], odd[m1 * R2 + t]), a.scale);
+        if (i < rows) row[i] = cscale(cadd(v[m1], odd.at(m1, t)), a.scale);
     }
 }
 
@@ -366,7 +388,7 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
     const LineBuf<T2> buf{sm + gid * LB, R2 + 1, 1};
     T2* own = sm + gid * LB;
     const T2* partner = sm + (gid ^ 1) * LB;
-    const T2* odd = sm + (gid + 2) * LB;
+    const LineBuf<T2> odd{sm + (gid + 2) * LB, R2 + 1, 1};
     const T2* ux = px ? a.ux1 : a.ux0;
     while (it < iters) {
         const int nxt = live(it + gridDim.x);
@@ -387,9 +409,9 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
         __syncthreads();  // the W rows are in registers: the next iteration's may come in
         if (tid == 0 && nxt < iters) issue(nxt, true, false);
         fwd_first<NP>(v, t, a.taP, buf);
-        __syncthreads();
+        __syncwarp();
         fwd_second<NP>(v, t, buf);
-        __syncthreads();  // the buffers are read; they now carry the spectra values to the partner
+        __syncwarp();  // the line's buffer is read; it now carries the spectra values to the partner
 #pragma unroll
         for (int q = 0; q < R1; ++q) own[q * R2 + t] = v[q];
         if (__syncthreads_or(!mbar_wait(&bar[1], done[1] & 1, a.fault))) break;
@@ -425,12 +447,11 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
         __syncthreads();  // the spectra and the partner values are read
         if (tid == 0 && nxt < iters) issue(nxt, false, true);
         inv_first<NP>(v, t, a.tbP, buf);
-        __syncthreads();
+        __syncwarp();
         inv_second<NP>(v, t, buf);
-        __syncthreads();
         if (px) {
 #pragma unroll
-            for (int m1 = 0; m1 < R1; ++m1) own[m1 * R2 + t] = cmulc(v[m1], __ldg(&a.modP[R2 * m1 + t]));
+            for (int m1 = 0; m1 < R1; ++m1) buf.at(m1, t) = cmulc(v[m1], __ldg(&a.modP[R2 * m1 + t]));
         }
         __syncthreads();
         if (!px) {
@@ -438,7 +459,7 @@ __global__ void __launch_bounds__(Fast<T>::threads, (MixShape<T, NP>::blocks)) k
 #pragma unroll
             for (int m1 = 0; m1 < R1; ++m1) {
                 const int i = R2 * m1 + t;
-                if (i < rows) row[i] = cscale(cadd(v[m1], odd[m1 * R2 + t]), a.scale);
+                if (i < rows) row[i] = cscale(cadd(v[m1], odd.at(m1, t)), a.scale);
             }
         }
         it = nxt;
