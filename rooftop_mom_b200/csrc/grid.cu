@@ -342,10 +342,10 @@ template <typename T> static GridArgs<T> product_args(const GridApplicator& g, S
     a.planQ = g.tQ->plan;
     if constexpr (sizeof(T) == 8) {
         a.twP = g.tP->tw64; a.twQ = g.tQ->tw64; a.modP = g.tP->mod64; a.modQ = g.tQ->mod64;
-        a.taP = g.tP->ta64; a.tbP = g.tP->tb64; a.taQ = g.tQ->ta64; a.tbQ = g.tQ->tb64;
+        a.taP = g.tP->ta64; a.t3P = g.tP->t364; a.t3Q = g.tQ->t364; a.tbP = g.tP->tb64; a.taQ = g.tQ->ta64; a.tbQ = g.tQ->tb64;
     } else {
         a.twP = g.tP->tw32; a.twQ = g.tQ->tw32; a.modP = g.tP->mod32; a.modQ = g.tQ->mod32;
-        a.taP = g.tP->ta32; a.tbP = g.tP->tb32; a.taQ = g.tQ->ta32; a.tbQ = g.tQ->tb32;
+        a.taP = g.tP->ta32; a.t3P = g.tP->t332; a.t3Q = g.tQ->t332; a.tbP = g.tP->tb32; a.taQ = g.tQ->ta32; a.tbQ = g.tQ->tb32;
     }
     a.spec = g.spec.as<T2>();
     a.mode = g.mode;

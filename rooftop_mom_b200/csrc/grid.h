@@ -24,7 +24,8 @@ namespace rtm {
 enum GridMode { kGen3 = 0, kBlock4 = 1, kStrip = 2 };
 
 // How the three kernels of a power-of-two split product run (grid_fast.cu): the CTAs an SM holds in
-// the y passes (the launch bound; 1 to 3, 3 for FP64 only) and the form of the x-mix. A product takes the
+// the y passes (the launch bound; 1 to 3, 3 for FP64 only) and the form of the x-mix. At the lengths that run in
+// three steps (grid_fast.cu), 1 CTA and kMixDirect1 stand for that form. A product takes the
 // schedule the autotuner measured best for its precision and transform grid (tune.cpp), or the rules of
 // default_fast_schedule when none was measured.
 enum MixKind { kMixDirect1 = 0, kMixDirect2 = 1, kMixDirect3 = 2, kMixPipelined = 3 };

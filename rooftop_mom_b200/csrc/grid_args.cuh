@@ -31,6 +31,8 @@ template <typename T> struct GridArgs {
     const T2* twQ;
     const T2* taP;  // the twiddles of power-of-two lengths' splits (FftTables)
     const T2* tbP;
+    const T2* t3P;  // the three-step twiddles of lines of P and Q (FftTables)
+    const T2* t3Q;
     const T2* taQ;
     const T2* tbQ;
     const T2* modP;

@@ -145,6 +145,148 @@ __device__ __forceinline__ void inv_second(T2 (&v)[Shape<N>::R1], int t, const L
     dft_reg<R1, true>(v);
 }
 
+// Lines in three steps, for N = R1 64 (R1 = 4, 8, 16): the TL threads of a line hold V = N / TL values of two transforms,
+// which share the twiddles. With r = 8 t1 + t0, k = k1 + R1 k2 + 8 R1 k3 and a buffer of elements (k1, r), the steps run
+// over units of R1, 8 and 8 points, a thread taking unit number thread + TL u:
+//   unit r            x[64 a + r]; DFT over a, twiddle wN^(r k1), written to (k1, r);
+//   unit 8 k1 + t0    reads (k1, 8 t1 + t0), DFT over t1, twiddle w64^(t0 k2), written back to (k1, 8 k2 + t0);
+//   unit k1 + R1 k2   reads (k1, 8 k2 + t0), DFT over t0: X[k], consecutive threads on consecutive frequencies.
+// The inverse runs backwards. Every thread writes where it has read, so a step needs one barrier, among its line's threads.
+// ES: the stride of the buffer's elements (lines of a CTA may be interleaved); its second transform lies LB ES further.
+template <typename T, int N, int ES> struct Lines3 {
+    using T2 = typename Cx<T>::T2;
+    static constexpr int R1 = N / 64;
+    static constexpr int V = R1 <= 8 ? 8 : R1, TL = N / V;  // values and threads a line
+    static constexpr int UA = 64 / TL, UB = V / 8;          // units a thread: first step, second and third
+    // Element (k1, 8 r1 + r0) at LS k1 + PK r1 + r0: the 8 (FP64) or 16 lanes that share a wavefront meet in different
+    // banks in the third step for every R1, and nearly so in the others.
+    static constexpr int PK = R1 == 4 ? 9 : 8, LS = R1 == 4 ? (sizeof(T) == 8 ? 74 : 76) : 65;
+    static constexpr int LB = R1 * LS;  // buffer elements of one transform
+    static constexpr int CS = LB * ES;
+
+    template <int R, bool INV> static __device__ __forceinline__ void dft(T2* v) {
+        if constexpr (R == 4) dft4<INV>(v[0], v[1], v[2], v[3]);
+        else if constexpr (R == 8) dft8<INV>(v);
+        else dft16<INV>(v);
+    }
+    // Value R1 u + e of a thread is element 64 e + tid + TL u of the line; transformed, value 8 u + k3 is frequency
+    // tid + TL u + 8 R1 k3.
+    static __device__ __forceinline__ int elem(int tid, int u, int e) { return 64 * e + tid + TL * u; }
+    static __device__ __forceinline__ int freq(int tid, int u, int k3) { return tid + TL * u + 8 * R1 * k3; }
+    static __device__ __forceinline__ T2* first(T2* buf, int tid) { return buf + (PK * (tid / 8) + tid % 8) * ES; }
+    static __device__ __forceinline__ T2* third(T2* buf, int tid) {
+        return buf + (LS * (tid % R1) + PK * (tid / R1)) * ES;
+    }
+
+    template <typename Sync>
+    static __device__ __forceinline__ void forward(T2 (&v)[2][V], int tid, T2* buf, const T2* __restrict__ t3, Sync sync) {
+        const T2* w64 = t3 + N;  // [k2][t0]
+#pragma unroll
+        for (int u = 0; u < UA; ++u) {
+            T2* at = first(buf, tid) + PK * (TL / 8) * u * ES;
+            dft<R1, false>(v[0] + R1 * u);
+            dft<R1, false>(v[1] + R1 * u);
+#pragma unroll
+            for (int k1 = 0; k1 < R1; ++k1) {
+                T2* d = at + LS * k1 * ES;
+                if (k1) {
+                    const T2 w = __ldg(&t3[64 * k1 + tid + TL * u]);
+                    d[0] = cmul(v[0][R1 * u + k1], w);
+                    d[CS] = cmul(v[1][R1 * u + k1], w);
+                } else {
+                    d[0] = v[0][R1 * u];
+                    d[CS] = v[1][R1 * u];
+                }
+            }
+        }
+        sync();
+        const int lo = tid % 8, mk = tid / 8;
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            const T2* mid = buf + (LS * (mk + TL / 8 * u) + lo) * ES;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[c][8 * u + e] = mid[c * CS + PK * e * ES];
+                dft<8, false>(v[c] + 8 * u);
+            }
+        }
+#pragma unroll
+        for (int k2 = 0; k2 < 8; ++k2) {
+            const T2 w = k2 ? __ldg(&w64[8 * k2 + lo]) : czero<T2>();
+#pragma unroll
+            for (int u = 0; u < UB; ++u) {
+                T2* d = buf + (LS * (mk + TL / 8 * u) + lo + PK * k2) * ES;
+                d[0] = k2 ? cmul(v[0][8 * u + k2], w) : v[0][8 * u];
+                d[CS] = k2 ? cmul(v[1][8 * u + k2], w) : v[1][8 * u];
+            }
+        }
+        sync();
+        const T2* own = third(buf, tid);
+#pragma unroll
+        for (int u = 0; u < UB; ++u)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[c][8 * u + e] = own[c * CS + (PK * (TL / R1) * u + e) * ES];
+                dft<8, false>(v[c] + 8 * u);
+            }
+    }
+
+    template <typename Sync>
+    static __device__ __forceinline__ void inverse(T2 (&v)[2][V], int tid, T2* buf, const T2* __restrict__ t3, Sync sync) {
+        const T2* w64 = t3 + N;
+        T2* own = third(buf, tid);
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            dft<8, true>(v[0] + 8 * u);
+            dft<8, true>(v[1] + 8 * u);
+            const int k2 = tid / R1 + TL / R1 * u;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                T2* d = own + (PK * (TL / R1) * u + e) * ES;
+                if (e) {
+                    const T2 w = __ldg(&w64[8 * k2 + e]);
+                    d[0] = cmulc(v[0][8 * u + e], w);
+                    d[CS] = cmulc(v[1][8 * u + e], w);
+                } else {
+                    d[0] = v[0][8 * u];
+                    d[CS] = v[1][8 * u];
+                }
+            }
+        }
+        sync();
+        const int lo = tid % 8, mk = tid / 8;
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            const int k1 = mk + TL / 8 * u;
+            T2* mid = buf + (LS * k1 + lo) * ES;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[c][8 * u + e] = mid[c * CS + PK * e * ES];
+                dft<8, true>(v[c] + 8 * u);
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const T2 w = __ldg(&t3[64 * k1 + 8 * e + lo]);
+                mid[PK * e * ES] = cmulc(v[0][8 * u + e], w);
+                mid[CS + PK * e * ES] = cmulc(v[1][8 * u + e], w);
+            }
+        }
+        sync();
+        const T2* at = first(buf, tid);
+#pragma unroll
+        for (int u = 0; u < UA; ++u)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                for (int k1 = 0; k1 < R1; ++k1) v[c][R1 * u + k1] = at[c * CS + (PK * (TL / 8) * u + LS * k1) * ES];
+                dft<R1, true>(v[c] + R1 * u);
+            }
+    }
+};
+
 // --------------------------------------------------------------------------------------------
 // y-forward: TI x-columns of one component; a group per (column, y subband). Thread index
 // l + TI (py + 2 t): consecutive threads take consecutive columns, so rows of TI elements are read
@@ -302,6 +444,111 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
         const int i = R2 * m1 + t;
         if (i < rows) row[i] = cscale(cadd(v[m1], odd.at(m1, t)), a.scale);
     }
+}
+
+// The x lines that run in three steps, a thread holding both components: they share the twiddles, the phases and E, and
+// meet in registers, and the small radices need half the registers. The L1 pipe bounds both forms (FP64 512 x 512 with
+// four vectors: 49 % busy at 8 warps an SM before, 70 % now). Product, two steps -> three: FP64 256 x 256 15.9 -> 14.2 us,
+// four vectors 42.9 -> 38.3; 512 x 512 46.6 -> 37.2 and 185 -> 152; FP32 512 x 512 29.6 -> 27.9 and 94 -> 81; 1024 x 1024
+// 104 -> 93 and 382 -> 350. FP32 256 x 256 stays on two steps (12.4 against 12.5 us, 23.4 against 24.9): its lines exchange
+// within their warps there; shorter lines leave too few threads for three steps.
+constexpr bool three_step(int n, bool fp64) { return fp64 ? n == 256 || n == 512 : n == 512 || n == 1024; }
+
+template <typename T, int NP> struct XMix3 {
+    using L = Lines3<T, NP, 1>;
+    static constexpr int threads = 128, teams = threads / (2 * L::TL);  // y frequencies a CTA
+    static constexpr int smem_elems = teams * 4 * L::LB;
+};
+
+template <typename T, int NP, int MINB>
+__global__ void __launch_bounds__((XMix3<T, NP>::threads), MINB) k_fast_x_mix_3(const GridArgs<T> a) {
+    using T2 = typename Cx<T>::T2;
+    using L = Lines3<T, NP, 1>;
+    constexpr int R1 = L::R1, TL = L::TL, LB = L::LB;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    griddep_wait();
+    const int py = blockIdx.y, rhs = blockIdx.z;
+    if (skipped(a, rhs)) return;
+    const PlateDesc<T> pd = plate_of(a, rhs);
+    const int tid = threadIdx.x % TL, line = threadIdx.x / TL, px = line % 2;
+    const int j = blockIdx.x * XMix3<T, NP>::teams + line / 2;  // Q is a power of two >= 32: no CTA is ragged
+    const int64_t QP = (int64_t)a.Q * NP;
+    T2* buf = reinterpret_cast<T2*>(smem_raw) + line * 2 * LB;
+    T2* row = a.work + (int64_t)rhs * a.work_rhs + (int64_t)(py * 2) * QP + (int64_t)j * NP;
+    auto sync = [line]() {
+        if constexpr (TL == 32) __syncwarp();
+        else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + line), "n"(TL) : "memory");
+    };
+    T2 v[2][L::V];
+#pragma unroll
+    for (int u = 0; u < L::UA; ++u)
+#pragma unroll
+        for (int e = 0; e < R1; ++e) {
+            const int i = L::elem(tid, u, e);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) v[c][R1 * u + e] = i < pd.rows[c] ? row[c * QP + i] : czero<T2>();
+            if (px) {
+                const T2 m = __ldg(&a.modP[i]);
+                v[0][R1 * u + e] = cmul(v[0][R1 * u + e], m);
+                v[1][R1 * u + e] = cmul(v[1][R1 * u + e], m);
+            }
+        }
+    L::forward(v, tid, buf, a.t3P, sync);
+    {
+        const T2* spec = pd.spec + (int64_t)((px + 2 * py) * 3) * QP + (int64_t)even_freq(j, py, a.Q) * NP;
+        const T2* ux = px ? a.ux1 : a.ux0;
+        const T2 vv = __ldg(&(py ? a.vy1 : a.vy0)[j]);
+        const T cv = (vv.x * vv.x + vv.y * vv.y) * pd.inv_b2;
+#pragma unroll
+        for (int u = 0; u < L::UB; ++u)
+#pragma unroll
+            for (int k3 = 0; k3 < 8; ++k3) {
+                const int k = L::freq(tid, u, k3), ke = even_freq(k, px, NP);
+                const T2 E = __ldg(&spec[ke]);
+                const T2 uu = __ldg(&ux[k]);
+                const T cu = (uu.x * uu.x + uu.y * uu.y) * pd.inv_a2;
+                // qc = -u conj(v) / (ab): XY = qc E, YX = conj(qc) E
+                T2 qc = cmulc(uu, vv);
+                qc.x = -qc.x * pd.inv_ab;
+                qc.y = -qc.y * pd.inv_ab;
+                const T2 me[2] = {v[0][8 * u + k3], v[1][8 * u + k3]};
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const T2 M = __ldg(&spec[(1 + c) * QP + ke]);
+                    const T cself = c ? cv : cu;
+                    // M me - cself E me + coupling E other = M me + E (coupling other - cself me)
+                    const T2 cp = cmul(c ? cconj(qc) : qc, me[1 - c]);
+                    const T2 d = make_vec2<T2>(cp.x - cself * me[c].x, cp.y - cself * me[c].y);
+                    v[c][8 * u + k3] = cadd(cmul(M, me[c]), cmul(E, d));
+                }
+            }
+    }
+    L::inverse(v, tid, buf, a.t3P, sync);
+    // the even subband's threads finish component 0 of the sum, the odd one's component 1
+    T2* mine = L::first(buf, tid) + (1 - px) * LB;
+#pragma unroll
+    for (int u = 0; u < L::UA; ++u)
+#pragma unroll
+        for (int e = 0; e < R1; ++e) {
+            const int o = R1 * u + e;
+            if (px) {
+                const T2 m = __ldg(&a.modP[L::elem(tid, u, e)]);
+                v[0][o] = cmulc(v[0][o], m);
+                v[1][o] = cmulc(v[1][o], m);
+            }
+            mine[L::PK * (TL / 8) * u + L::LS * e] = px ? v[0][o] : v[1][o];
+        }
+    __syncthreads();
+    const T2* theirs = L::first(reinterpret_cast<T2*>(smem_raw) + (line ^ 1) * 2 * LB, tid) + px * LB;
+#pragma unroll
+    for (int u = 0; u < L::UA; ++u)
+#pragma unroll
+        for (int e = 0; e < R1; ++e) {
+            const int i = L::elem(tid, u, e), o = R1 * u + e;
+            const T2 got = theirs[L::PK * (TL / 8) * u + L::LS * e];
+            const T2 even = px ? got : v[0][o], odd = px ? v[1][o] : got;
+            if (i < pd.rows[px]) row[px * QP + i] = cscale(cadd(even, odd), a.scale);
+        }
 }
 
 // x-mix, pipelined form: persistent CTAs. A CTA takes the iterations it = blockIdx.x, blockIdx.x + gridDim.x, ...; an
@@ -516,6 +763,99 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_y_inv(const Gri
     }
 }
 
+// The y passes in three steps: a thread holds both subbands of a column, which share its loads and twiddles and, in the
+// inverse, sum in registers. TI columns a CTA, interleaved in the buffer: thread l + TI tid.
+template <typename T, int NQ> struct Y3 {
+    static constexpr int TI = 64 / sizeof(typename Cx<T>::T2);
+    using L = Lines3<T, NQ, TI>;
+    static constexpr int threads = TI * L::TL;
+    static constexpr size_t smem = (size_t)2 * L::CS * sizeof(typename Cx<T>::T2);
+};
+
+struct CtaSync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+
+template <typename T, int NQ, int MINB>
+__global__ void __launch_bounds__((Y3<T, NQ>::threads), MINB)
+    k_fast_y_fwd_3(const GridArgs<T> a, const typename Cx<T>::T2* __restrict__ x) {
+    using T2 = typename Cx<T>::T2;
+    using L = typename Y3<T, NQ>::L;
+    constexpr int R1 = L::R1, TI = Y3<T, NQ>::TI;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    griddep_wait();
+    const int c = blockIdx.y, rhs = blockIdx.z;
+    if (skipped(a, rhs)) return;
+    const PlateDesc<T> pd = plate_of(a, rhs);
+    const int rows = pd.rows[c], cols = pd.cols[c];
+    if ((int)blockIdx.x * TI >= rows) return;  // a smaller plate of a batch
+    const int l = threadIdx.x % TI, tid = threadIdx.x / TI;
+    const int i = blockIdx.x * TI + l;
+    const bool on = i < rows;
+    const T2* xr = x + (int64_t)rhs * a.n + pd.off[c] + i;
+    T2 v[2][L::V];
+#pragma unroll
+    for (int u = 0; u < L::UA; ++u)
+#pragma unroll
+        for (int e = 0; e < R1; ++e) {
+            const int j = L::elem(tid, u, e);
+            v[0][R1 * u + e] = (on && j < cols) ? xr[(int64_t)j * rows] : czero<T2>();
+        }
+#pragma unroll
+    for (int u = 0; u < L::UA; ++u)
+#pragma unroll
+        for (int e = 0; e < R1; ++e) v[1][R1 * u + e] = cmul(v[0][R1 * u + e], __ldg(&a.modQ[L::elem(tid, u, e)]));
+    L::forward(v, tid, reinterpret_cast<T2*>(smem_raw) + l, a.t3Q, CtaSync{});
+    if (!on) return;
+    const int64_t QP = (int64_t)NQ * a.P;
+    T2* dst = a.work + (int64_t)rhs * a.work_rhs + c * QP + i;
+#pragma unroll
+    for (int py = 0; py < 2; ++py)
+#pragma unroll
+        for (int u = 0; u < L::UB; ++u)
+#pragma unroll
+            for (int k3 = 0; k3 < 8; ++k3) dst[2 * py * QP + (int64_t)L::freq(tid, u, k3) * a.P] = v[py][8 * u + k3];
+}
+
+template <typename T, int NQ, int MINB>
+__global__ void __launch_bounds__((Y3<T, NQ>::threads), MINB)
+    k_fast_y_inv_3(const GridArgs<T> a, typename Cx<T>::T2* __restrict__ y) {
+    using T2 = typename Cx<T>::T2;
+    using L = typename Y3<T, NQ>::L;
+    constexpr int R1 = L::R1, TI = Y3<T, NQ>::TI;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    griddep_wait();
+    const int c = blockIdx.y, rhs = blockIdx.z;
+    if (skipped(a, rhs)) return;
+    const PlateDesc<T> pd = plate_of(a, rhs);
+    const int rows = pd.rows[c], cols = pd.cols[c];
+    if ((int)blockIdx.x * TI >= rows) return;  // a smaller plate of a batch
+    const int l = threadIdx.x % TI, tid = threadIdx.x / TI;
+    const int i = blockIdx.x * TI + l;
+    const bool on = i < rows;
+    const int64_t QP = (int64_t)NQ * a.P;
+    const T2* src = a.work + (int64_t)rhs * a.work_rhs + c * QP + (on ? i : 0);
+    T2 v[2][L::V];
+#pragma unroll
+    for (int py = 0; py < 2; ++py)
+#pragma unroll
+        for (int u = 0; u < L::UB; ++u)
+#pragma unroll
+            for (int k3 = 0; k3 < 8; ++k3)
+                v[py][8 * u + k3] = on ? src[2 * py * QP + (int64_t)L::freq(tid, u, k3) * a.P] : czero<T2>();
+    L::inverse(v, tid, reinterpret_cast<T2*>(smem_raw) + l, a.t3Q, CtaSync{});
+    if (!on) return;
+    T2* yr = y + (int64_t)rhs * a.n + pd.off[c] + i;
+#pragma unroll
+    for (int u = 0; u < L::UA; ++u)
+#pragma unroll
+        for (int e = 0; e < R1; ++e) {
+            const int j = L::elem(tid, u, e), o = R1 * u + e;
+            const T2 odd = cmulc(v[1][o], __ldg(&a.modQ[j]));
+            if (j < cols) yr[(int64_t)j * rows] = cadd(v[0][o], odd);
+        }
+}
+
 template <typename T, int NQ> size_t y_smem() {
     constexpr int R1 = Shape<NQ>::R1, R2 = Shape<NQ>::R2, TI = Fast<T>::threads / (2 * R2);
     return (size_t)2 * TI * R1 * (R2 + 1) * sizeof(typename Cx<T>::T2);
@@ -543,9 +883,34 @@ template <typename T, int NQ, int MINB> int launch_y_b(const GridArgs<T>& a, int
     return RTM_OK;
 }
 
+template <typename T, int NQ> int launch_y_3(const GridArgs<T>& a, int nrhs, const void* x, void* y, bool fwd,
+                                             cudaStream_t s) {
+    using T2 = typename Cx<T>::T2;
+    using S = Y3<T, NQ>;
+    constexpr int MINB = sizeof(T) == 8 ? (NQ == 256 ? 3 : 2) : (NQ == 1024 ? 1 : 2);
+    static DeviceOnce once;
+    RTM_TRY(once([]() -> int {
+        RTM_CUDA(cudaFuncSetAttribute(k_fast_y_fwd_3<T, NQ, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem));
+        RTM_CUDA(cudaFuncSetAttribute(k_fast_y_inv_3<T, NQ, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem));
+        return RTM_OK;
+    }));
+    const int rows_max = a.rows[0] > a.rows[1] ? a.rows[0] : a.rows[1];
+    const dim3 grid((rows_max + S::TI - 1) / S::TI, 2, nrhs);
+    if (fwd)
+        RTM_CUDA(launch_dependent(k_fast_y_fwd_3<T, NQ, MINB>, grid, dim3(S::threads), S::smem, s, a,
+                                  static_cast<const T2*>(x)));
+    else
+        RTM_CUDA(launch_dependent(k_fast_y_inv_3<T, NQ, MINB>, grid, dim3(S::threads), S::smem, s, a, static_cast<T2*>(y)));
+    count_launch();
+    return RTM_OK;
+}
+
 template <typename T, int NQ> int launch_y(const GridArgs<T>& a, int nrhs, const void* x, void* y, bool fwd,
                                            int minb, cudaStream_t s) {
-    if (minb <= 1) return launch_y_b<T, NQ, 1>(a, nrhs, x, y, fwd, s);
+    if (minb <= 1) {
+        if constexpr (three_step(NQ, sizeof(T) == 8)) return launch_y_3<T, NQ>(a, nrhs, x, y, fwd, s);
+        else return launch_y_b<T, NQ, 1>(a, nrhs, x, y, fwd, s);
+    }
     if constexpr (sizeof(T) == 8) {
         if (minb >= 3) return launch_y_b<T, NQ, 3>(a, nrhs, x, y, fwd, s);
     }
@@ -568,6 +933,22 @@ template <typename T, int NP, int MINB> int launch_x_direct(const GridArgs<T>& a
     }));
     const dim3 grid((a.Q + TEAMS - 1) / TEAMS, 2, nrhs);
     RTM_CUDA(launch_dependent(k_fast_x_mix_direct<T, NP, MINB>, grid, dim3(Fast<T>::threads), smem, s, a));
+    count_launch();
+    return RTM_OK;
+}
+
+template <typename T, int NP> int launch_x_3(const GridArgs<T>& a, int nrhs, cudaStream_t s) {
+    using S = XMix3<T, NP>;
+    // CTAs an SM, one less and one more: FP64 2 (512 x 512 product 37.2 us, with 3 or 4 spills: 40.4, 37.6), FP32 512
+    // 4 (27.9; 5: 28.3), FP32 1024 3 (alone 93; 2: 98, 4: 105).
+    constexpr int MINB = sizeof(T) == 8 ? 2 : NP == 1024 ? 3 : 4;
+    const size_t smem = (size_t)S::smem_elems * sizeof(typename Cx<T>::T2);
+    static DeviceOnce once;
+    RTM_TRY(once([smem]() -> int {
+        RTM_CUDA(cudaFuncSetAttribute(k_fast_x_mix_3<T, NP, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        return RTM_OK;
+    }));
+    RTM_CUDA(launch_dependent(k_fast_x_mix_3<T, NP, MINB>, dim3(a.Q / S::teams, 2, nrhs), dim3(S::threads), smem, s, a));
     count_launch();
     return RTM_OK;
 }
@@ -602,7 +983,8 @@ template <typename T, int NP> int launch_x(const GridArgs<T>& a, int nrhs, int k
     if constexpr (sizeof(T) == 8) {
         if (kind == kMixDirect3) return launch_x_direct<T, NP, 3>(a, nrhs, s);
     }
-    return launch_x_direct<T, NP, 1>(a, nrhs, s);
+    if constexpr (three_step(NP, sizeof(T) == 8)) return launch_x_3<T, NP>(a, nrhs, s);
+    else return launch_x_direct<T, NP, 1>(a, nrhs, s);
 }
 
 template <typename T> int dispatch_y(const GridArgs<T>& a, int nrhs, const void* x, void* y, bool fwd, int minb,
@@ -641,14 +1023,10 @@ bool fast_split_eligible(int P, int Q, bool fp64) {
 
 FastSchedule default_fast_schedule(int P, int Q, bool fp64) {
     FastSchedule f;
-    // y passes: FP32 two CTAs of 256 threads an SM (128 registers, no spills up to lines of 1024); FP64
-    // three CTAs of 128 threads below lines of 512, two at 512 (up to 255 registers).
-    f.y_blocks = fp64 ? (Q >= 512 ? 2 : 3) : 2;
-    // x-mix: the pipelined form at FP32 1024 (one CTA of 256 threads an SM either way, and 100 MB of spectra
-    // that do not stay in L2 between products); elsewhere the direct form, which keeps more warps resident.
-    if (!fp64 && P >= 1024) f.x_kind = kMixPipelined;
-    else if (fp64) f.x_kind = P >= 512 ? kMixDirect1 : kMixDirect3;
-    else f.x_kind = kMixDirect2;
+    // Three steps where the lengths have them; else the y passes take FP32 two CTAs of 256 threads an SM (128 registers),
+    // FP64 three of 128, and the x-mix the direct form, which keeps more warps resident than the pipelined one.
+    f.y_blocks = three_step(Q, fp64) ? 1 : fp64 ? 3 : 2;
+    f.x_kind = three_step(P, fp64) ? kMixDirect1 : fp64 ? kMixDirect3 : kMixDirect2;
     return f;
 }
 

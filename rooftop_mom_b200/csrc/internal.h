@@ -149,6 +149,9 @@ struct FftTables {
     const double2* tb64;
     const float2* ta32;
     const float2* tb32;
+    // Lengths n >= 256, for the three-step lines of grid_fast.cu: w_n^(t k1) at 64 k1 + t, then w_64^(t0 k2) at 8 k2 + t0.
+    const double2* t364;
+    const float2* t332;
     const double2* tw64;   // n entries
     const float2* tw32;
     const double2* mod64;  // exp(-i pi d / n), d < n (the odd-subband modulation)

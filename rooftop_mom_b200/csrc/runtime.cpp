@@ -494,21 +494,32 @@ int fft_tables(int n, const FftTables** out) {
         rp.kern32 = rp.chirp32 + n;
     }
     if (rp.n1 && n >= 32 && (n & (n - 1)) == 0) {
-        std::vector<double2> t64((size_t)2 * n);
+        const int r1 = n / 64, extra = n >= 256 ? n + 64 : 0;
+        std::vector<double2> t64((size_t)2 * n + extra);
         for (int k1 = 0; k1 < rp.n1; ++k1)
             for (int t = 0; t < rp.n2; ++t) t64[k1 * rp.n2 + t] = t64[n + t * rp.n1 + k1] = tw[t * k1];
-        std::vector<float2> t32((size_t)2 * n);
-        for (int i = 0; i < 2 * n; ++i) t32[i] = make_float2((float)t64[i].x, (float)t64[i].y);
+        if (extra) {
+            for (int k1 = 0; k1 < r1; ++k1)
+                for (int t = 0; t < 64; ++t) t64[2 * n + 64 * k1 + t] = tw[t * k1];
+            for (int k2 = 0; k2 < 8; ++k2)
+                for (int t0 = 0; t0 < 8; ++t0) t64[3 * n + 8 * k2 + t0] = tw[r1 * t0 * k2];
+        }
+        std::vector<float2> t32(t64.size());
+        for (size_t i = 0; i < t32.size(); ++i) t32[i] = make_float2((float)t64[i].x, (float)t64[i].y);
         void* mem = nullptr;
-        RTM_CUDA(cudaMalloc(&mem, 2 * (size_t)n * (sizeof(double2) + sizeof(float2))));
+        RTM_CUDA(cudaMalloc(&mem, t64.size() * (sizeof(double2) + sizeof(float2))));
         double2* d64 = (double2*)mem;
-        float2* d32 = (float2*)(d64 + 2 * n);
+        float2* d32 = (float2*)(d64 + t64.size());
         RTM_CUDA(cudaMemcpy(d64, t64.data(), t64.size() * sizeof(double2), cudaMemcpyHostToDevice));
         RTM_CUDA(cudaMemcpy(d32, t32.data(), t32.size() * sizeof(float2), cudaMemcpyHostToDevice));
         e.t.ta64 = d64;
         e.t.tb64 = d64 + n;
         e.t.ta32 = d32;
         e.t.tb32 = d32 + n;
+        if (extra) {
+            e.t.t364 = d64 + 2 * n;
+            e.t.t332 = d32 + 2 * n;
+        }
     }
     auto res = g_tables.emplace(TableKey{dev, n}, e);
     *out = &res.first->second.t;
