@@ -362,6 +362,8 @@ template <typename T> static GridArgs<T> product_args(const GridApplicator& g, S
 template <typename T>
 static int reg_pass(int pass, const GridArgs<T>& a, const RegPlan& r, int nrhs, const void* x, void* y, cudaStream_t s) {
     const bool wide = r.n1 > 16;
+    if (a.npy == a.nsy && a.nsx == a.nsy && three_step_length(pass == kRegXMix ? a.P : a.Q, sizeof(T) == 8))
+        return launch_three_step<T>(pass, a, nrhs, x, y, s);
     if (r.m != r.n)  // FP32 lines transform in FP64 there
         return wide ? launch_reg_pass<T, double, 1, true>(pass, a, r, nrhs, x, y, s)
                     : launch_reg_pass<T, double, 0, true>(pass, a, r, nrhs, x, y, s);

@@ -86,4 +86,9 @@ enum RegPass { kRegYFwd = 0, kRegXMix = 1, kRegYInv = 2 };
 template <typename T, typename C, int CLS, bool BLUE>
 int launch_reg_pass(int pass, GridArgs<T> a, const RegPlan& r, int nrhs, const void* x, void* y, cudaStream_t s);
 
+// One pass of a product of grid_reg.cu whose lines run in three steps (grid_fast.cu): both subbands or none in a launch.
+bool three_step_length(int n, bool fp64);
+template <typename T>
+int launch_three_step(int pass, const GridArgs<T>& a, int nrhs, const void* x, void* y, cudaStream_t s);
+
 }  // namespace rtm

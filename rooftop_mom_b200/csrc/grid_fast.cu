@@ -454,14 +454,15 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
 // within their warps there; shorter lines leave too few threads for three steps.
 constexpr bool three_step(int n, bool fp64) { return fp64 ? n == 256 || n == 512 : n == 512 || n == 1024; }
 
-template <typename T, int NP> struct XMix3 {
+// SUB: the subbands along x (2: a split product, 1: an embedding or a circulant).
+template <typename T, int NP, int SUB> struct XMix3 {
     using L = Lines3<T, NP, 1>;
-    static constexpr int threads = 128, teams = threads / (2 * L::TL);  // y frequencies a CTA
-    static constexpr int smem_elems = teams * 4 * L::LB;
+    static constexpr int threads = 128, teams = threads / (SUB * L::TL);  // y frequencies a CTA
+    static constexpr int smem_elems = teams * SUB * 2 * L::LB;
 };
 
-template <typename T, int NP, int MINB>
-__global__ void __launch_bounds__((XMix3<T, NP>::threads), MINB) k_fast_x_mix_3(const GridArgs<T> a) {
+template <typename T, int NP, int SUB, int MINB>
+__global__ void __launch_bounds__((XMix3<T, NP, SUB>::threads), MINB) k_fast_x_mix_3(const GridArgs<T> a) {
     using T2 = typename Cx<T>::T2;
     using L = Lines3<T, NP, 1>;
     constexpr int R1 = L::R1, TL = L::TL, LB = L::LB;
@@ -470,11 +471,12 @@ __global__ void __launch_bounds__((XMix3<T, NP>::threads), MINB) k_fast_x_mix_3(
     const int py = blockIdx.y, rhs = blockIdx.z;
     if (skipped(a, rhs)) return;
     const PlateDesc<T> pd = plate_of(a, rhs);
-    const int tid = threadIdx.x % TL, line = threadIdx.x / TL, px = line % 2;
-    const int j = blockIdx.x * XMix3<T, NP>::teams + line / 2;  // Q is a power of two >= 32: no CTA is ragged
+    const int tid = threadIdx.x % TL, line = threadIdx.x / TL, px = SUB == 2 ? line % 2 : 0;
+    const int j = blockIdx.x * XMix3<T, NP, SUB>::teams + line / SUB;
+    const bool on = j < a.Q;
     const int64_t QP = (int64_t)a.Q * NP;
     T2* buf = reinterpret_cast<T2*>(smem_raw) + line * 2 * LB;
-    T2* row = a.work + (int64_t)rhs * a.work_rhs + (int64_t)(py * 2) * QP + (int64_t)j * NP;
+    T2* row = a.work + (int64_t)rhs * a.work_rhs + (int64_t)(py * 2) * QP + (int64_t)(on ? j : 0) * NP;
     auto sync = [line]() {
         if constexpr (TL == 32) __syncwarp();
         else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + line), "n"(TL) : "memory");
@@ -486,7 +488,7 @@ __global__ void __launch_bounds__((XMix3<T, NP>::threads), MINB) k_fast_x_mix_3(
         for (int e = 0; e < R1; ++e) {
             const int i = L::elem(tid, u, e);
 #pragma unroll
-            for (int c = 0; c < 2; ++c) v[c][R1 * u + e] = i < pd.rows[c] ? row[c * QP + i] : czero<T2>();
+            for (int c = 0; c < 2; ++c) v[c][R1 * u + e] = on && i < pd.rows[c] ? row[c * QP + i] : czero<T2>();
             if (px) {
                 const T2 m = __ldg(&a.modP[i]);
                 v[0][R1 * u + e] = cmul(v[0][R1 * u + e], m);
@@ -494,10 +496,23 @@ __global__ void __launch_bounds__((XMix3<T, NP>::threads), MINB) k_fast_x_mix_3(
             }
         }
     L::forward(v, tid, buf, a.t3P, sync);
-    {
-        const T2* spec = pd.spec + (int64_t)((px + 2 * py) * 3) * QP + (int64_t)even_freq(j, py, a.Q) * NP;
+    if (SUB == 1 && a.mode == kBlock4) {
+        // blocks XX, XY, YX, YY
+        const T2* spec = pd.spec + (int64_t)(on ? j : 0) * NP;
+#pragma unroll
+        for (int u = 0; u < L::UB; ++u)
+#pragma unroll
+            for (int k3 = 0; k3 < 8; ++k3) {
+                const int k = L::freq(tid, u, k3);
+                const T2 mx = v[0][8 * u + k3], my = v[1][8 * u + k3];
+                v[0][8 * u + k3] = cadd(cmul(__ldg(&spec[k]), mx), cmul(__ldg(&spec[QP + k]), my));
+                v[1][8 * u + k3] = cadd(cmul(__ldg(&spec[3 * QP + k]), my), cmul(__ldg(&spec[2 * QP + k]), mx));
+            }
+    } else {
+        const int jc = on ? j : 0;
+        const T2* spec = pd.spec + (int64_t)((px + SUB * py) * 3) * QP + (int64_t)even_freq(jc, py, a.Q) * NP;
         const T2* ux = px ? a.ux1 : a.ux0;
-        const T2 vv = __ldg(&(py ? a.vy1 : a.vy0)[j]);
+        const T2 vv = __ldg(&(py ? a.vy1 : a.vy0)[jc]);
         const T cv = (vv.x * vv.x + vv.y * vv.y) * pd.inv_b2;
 #pragma unroll
         for (int u = 0; u < L::UB; ++u)
@@ -524,6 +539,19 @@ __global__ void __launch_bounds__((XMix3<T, NP>::threads), MINB) k_fast_x_mix_3(
             }
     }
     L::inverse(v, tid, buf, a.t3P, sync);
+    if constexpr (SUB == 1) {
+        if (!on) return;
+#pragma unroll
+        for (int u = 0; u < L::UA; ++u)
+#pragma unroll
+            for (int e = 0; e < R1; ++e) {
+                const int i = L::elem(tid, u, e);
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    if (i < pd.rows[c]) row[c * QP + i] = cscale(v[c][R1 * u + e], a.scale);
+            }
+        return;
+    }
     // the even subband's threads finish component 0 of the sum, the odd one's component 1
     T2* mine = L::first(buf, tid) + (1 - px) * LB;
 #pragma unroll
@@ -539,6 +567,7 @@ __global__ void __launch_bounds__((XMix3<T, NP>::threads), MINB) k_fast_x_mix_3(
             mine[L::PK * (TL / 8) * u + L::LS * e] = px ? v[0][o] : v[1][o];
         }
     __syncthreads();
+    if (!on) return;
     const T2* theirs = L::first(reinterpret_cast<T2*>(smem_raw) + (line ^ 1) * 2 * LB, tid) + px * LB;
 #pragma unroll
     for (int u = 0; u < L::UA; ++u)
@@ -764,7 +793,8 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_y_inv(const Gri
 }
 
 // The y passes in three steps: a thread holds both subbands of a column, which share its loads and twiddles and, in the
-// inverse, sum in registers. TI columns a CTA, interleaved in the buffer: thread l + TI tid.
+// inverse, sum in registers; without subbands (SUB = 1) two columns TI apart. TI columns a CTA, interleaved in the buffer:
+// thread l + TI tid.
 template <typename T, int NQ> struct Y3 {
     static constexpr int TI = 64 / sizeof(typename Cx<T>::T2);
     using L = Lines3<T, NQ, TI>;
@@ -776,7 +806,7 @@ struct CtaSync {
     __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
 
-template <typename T, int NQ, int MINB>
+template <typename T, int NQ, int SUB, int MINB>
 __global__ void __launch_bounds__((Y3<T, NQ>::threads), MINB)
     k_fast_y_fwd_3(const GridArgs<T> a, const typename Cx<T>::T2* __restrict__ x) {
     using T2 = typename Cx<T>::T2;
@@ -788,10 +818,11 @@ __global__ void __launch_bounds__((Y3<T, NQ>::threads), MINB)
     if (skipped(a, rhs)) return;
     const PlateDesc<T> pd = plate_of(a, rhs);
     const int rows = pd.rows[c], cols = pd.cols[c];
-    if ((int)blockIdx.x * TI >= rows) return;  // a smaller plate of a batch
+    if ((int)blockIdx.x * TI * (3 - SUB) >= rows) return;  // a smaller plate of a batch
     const int l = threadIdx.x % TI, tid = threadIdx.x / TI;
-    const int i = blockIdx.x * TI + l;
-    const bool on = i < rows;
+    const int i = blockIdx.x * TI * (3 - SUB) + l;
+    // the second transform: the odd subband of the column, or the column TI further
+    const bool on = i < rows, on2 = SUB == 1 && i + TI < rows;
     const T2* xr = x + (int64_t)rhs * a.n + pd.off[c] + i;
     T2 v[2][L::V];
 #pragma unroll
@@ -800,24 +831,30 @@ __global__ void __launch_bounds__((Y3<T, NQ>::threads), MINB)
         for (int e = 0; e < R1; ++e) {
             const int j = L::elem(tid, u, e);
             v[0][R1 * u + e] = (on && j < cols) ? xr[(int64_t)j * rows] : czero<T2>();
+            if (SUB == 1) v[1][R1 * u + e] = (on2 && j < cols) ? xr[(int64_t)j * rows + TI] : czero<T2>();
         }
+    if (SUB == 2) {
 #pragma unroll
     for (int u = 0; u < L::UA; ++u)
 #pragma unroll
         for (int e = 0; e < R1; ++e) v[1][R1 * u + e] = cmul(v[0][R1 * u + e], __ldg(&a.modQ[L::elem(tid, u, e)]));
+    }
     L::forward(v, tid, reinterpret_cast<T2*>(smem_raw) + l, a.t3Q, CtaSync{});
     if (!on) return;
     const int64_t QP = (int64_t)NQ * a.P;
+    const int64_t second = SUB == 2 ? 2 * QP : TI;
     T2* dst = a.work + (int64_t)rhs * a.work_rhs + c * QP + i;
 #pragma unroll
-    for (int py = 0; py < 2; ++py)
+    for (int h = 0; h < 2; ++h) {
+        if (SUB == 1 && h && !on2) return;
 #pragma unroll
         for (int u = 0; u < L::UB; ++u)
 #pragma unroll
-            for (int k3 = 0; k3 < 8; ++k3) dst[2 * py * QP + (int64_t)L::freq(tid, u, k3) * a.P] = v[py][8 * u + k3];
+            for (int k3 = 0; k3 < 8; ++k3) dst[h * second + (int64_t)L::freq(tid, u, k3) * a.P] = v[h][8 * u + k3];
+    }
 }
 
-template <typename T, int NQ, int MINB>
+template <typename T, int NQ, int SUB, int MINB>
 __global__ void __launch_bounds__((Y3<T, NQ>::threads), MINB)
     k_fast_y_inv_3(const GridArgs<T> a, typename Cx<T>::T2* __restrict__ y) {
     using T2 = typename Cx<T>::T2;
@@ -829,20 +866,23 @@ __global__ void __launch_bounds__((Y3<T, NQ>::threads), MINB)
     if (skipped(a, rhs)) return;
     const PlateDesc<T> pd = plate_of(a, rhs);
     const int rows = pd.rows[c], cols = pd.cols[c];
-    if ((int)blockIdx.x * TI >= rows) return;  // a smaller plate of a batch
+    if ((int)blockIdx.x * TI * (3 - SUB) >= rows) return;  // a smaller plate of a batch
     const int l = threadIdx.x % TI, tid = threadIdx.x / TI;
-    const int i = blockIdx.x * TI + l;
-    const bool on = i < rows;
+    const int i = blockIdx.x * TI * (3 - SUB) + l;
+    // the second transform: the odd subband of the column, or the column TI further
+    const bool on = i < rows, on2 = SUB == 1 && i + TI < rows;
     const int64_t QP = (int64_t)NQ * a.P;
+    const int64_t second = SUB == 2 ? 2 * QP : TI;
     const T2* src = a.work + (int64_t)rhs * a.work_rhs + c * QP + (on ? i : 0);
     T2 v[2][L::V];
 #pragma unroll
-    for (int py = 0; py < 2; ++py)
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int u = 0; u < L::UB; ++u)
 #pragma unroll
             for (int k3 = 0; k3 < 8; ++k3)
-                v[py][8 * u + k3] = on ? src[2 * py * QP + (int64_t)L::freq(tid, u, k3) * a.P] : czero<T2>();
+                v[h][8 * u + k3] =
+                    (SUB == 1 && h ? on2 : on) ? src[h * second + (int64_t)L::freq(tid, u, k3) * a.P] : czero<T2>();
     L::inverse(v, tid, reinterpret_cast<T2*>(smem_raw) + l, a.t3Q, CtaSync{});
     if (!on) return;
     T2* yr = y + (int64_t)rhs * a.n + pd.off[c] + i;
@@ -851,8 +891,13 @@ __global__ void __launch_bounds__((Y3<T, NQ>::threads), MINB)
 #pragma unroll
         for (int e = 0; e < R1; ++e) {
             const int j = L::elem(tid, u, e), o = R1 * u + e;
-            const T2 odd = cmulc(v[1][o], __ldg(&a.modQ[j]));
-            if (j < cols) yr[(int64_t)j * rows] = cadd(v[0][o], odd);
+            if (SUB == 2) {
+                const T2 odd = cmulc(v[1][o], __ldg(&a.modQ[j]));
+                if (j < cols) yr[(int64_t)j * rows] = cadd(v[0][o], odd);
+            } else {
+                if (j < cols) yr[(int64_t)j * rows] = v[0][o];
+                if (on2 && j < cols) yr[(int64_t)j * rows + TI] = v[1][o];
+            }
         }
 }
 
@@ -883,24 +928,25 @@ template <typename T, int NQ, int MINB> int launch_y_b(const GridArgs<T>& a, int
     return RTM_OK;
 }
 
-template <typename T, int NQ> int launch_y_3(const GridArgs<T>& a, int nrhs, const void* x, void* y, bool fwd,
+template <typename T, int NQ, int SUB> int launch_y_3(const GridArgs<T>& a, int nrhs, const void* x, void* y, bool fwd,
                                              cudaStream_t s) {
     using T2 = typename Cx<T>::T2;
     using S = Y3<T, NQ>;
     constexpr int MINB = sizeof(T) == 8 ? (NQ == 256 ? 3 : 2) : (NQ == 1024 ? 1 : 2);
     static DeviceOnce once;
     RTM_TRY(once([]() -> int {
-        RTM_CUDA(cudaFuncSetAttribute(k_fast_y_fwd_3<T, NQ, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem));
-        RTM_CUDA(cudaFuncSetAttribute(k_fast_y_inv_3<T, NQ, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem));
+        RTM_CUDA(cudaFuncSetAttribute(k_fast_y_fwd_3<T, NQ, SUB, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem));
+        RTM_CUDA(cudaFuncSetAttribute(k_fast_y_inv_3<T, NQ, SUB, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem));
         return RTM_OK;
     }));
     const int rows_max = a.rows[0] > a.rows[1] ? a.rows[0] : a.rows[1];
-    const dim3 grid((rows_max + S::TI - 1) / S::TI, 2, nrhs);
+    constexpr int columns = S::TI * (3 - SUB);
+    const dim3 grid((rows_max + columns - 1) / columns, 2, nrhs);
     if (fwd)
-        RTM_CUDA(launch_dependent(k_fast_y_fwd_3<T, NQ, MINB>, grid, dim3(S::threads), S::smem, s, a,
+        RTM_CUDA(launch_dependent(k_fast_y_fwd_3<T, NQ, SUB, MINB>, grid, dim3(S::threads), S::smem, s, a,
                                   static_cast<const T2*>(x)));
     else
-        RTM_CUDA(launch_dependent(k_fast_y_inv_3<T, NQ, MINB>, grid, dim3(S::threads), S::smem, s, a, static_cast<T2*>(y)));
+        RTM_CUDA(launch_dependent(k_fast_y_inv_3<T, NQ, SUB, MINB>, grid, dim3(S::threads), S::smem, s, a, static_cast<T2*>(y)));
     count_launch();
     return RTM_OK;
 }
@@ -908,7 +954,7 @@ template <typename T, int NQ> int launch_y_3(const GridArgs<T>& a, int nrhs, con
 template <typename T, int NQ> int launch_y(const GridArgs<T>& a, int nrhs, const void* x, void* y, bool fwd,
                                            int minb, cudaStream_t s) {
     if (minb <= 1) {
-        if constexpr (three_step(NQ, sizeof(T) == 8)) return launch_y_3<T, NQ>(a, nrhs, x, y, fwd, s);
+        if constexpr (three_step(NQ, sizeof(T) == 8)) return launch_y_3<T, NQ, 2>(a, nrhs, x, y, fwd, s);
         else return launch_y_b<T, NQ, 1>(a, nrhs, x, y, fwd, s);
     }
     if constexpr (sizeof(T) == 8) {
@@ -937,18 +983,18 @@ template <typename T, int NP, int MINB> int launch_x_direct(const GridArgs<T>& a
     return RTM_OK;
 }
 
-template <typename T, int NP> int launch_x_3(const GridArgs<T>& a, int nrhs, cudaStream_t s) {
-    using S = XMix3<T, NP>;
+template <typename T, int NP, int SUB> int launch_x_3(const GridArgs<T>& a, int nrhs, cudaStream_t s) {
+    using S = XMix3<T, NP, SUB>;
     // CTAs an SM, one less and one more: FP64 2 (512 x 512 product 37.2 us, with 3 or 4 spills: 40.4, 37.6), FP32 512
     // 4 (27.9; 5: 28.3), FP32 1024 3 (alone 93; 2: 98, 4: 105).
     constexpr int MINB = sizeof(T) == 8 ? 2 : NP == 1024 ? 3 : 4;
     const size_t smem = (size_t)S::smem_elems * sizeof(typename Cx<T>::T2);
     static DeviceOnce once;
     RTM_TRY(once([smem]() -> int {
-        RTM_CUDA(cudaFuncSetAttribute(k_fast_x_mix_3<T, NP, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        RTM_CUDA(cudaFuncSetAttribute(k_fast_x_mix_3<T, NP, SUB, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         return RTM_OK;
     }));
-    RTM_CUDA(launch_dependent(k_fast_x_mix_3<T, NP, MINB>, dim3(a.Q / S::teams, 2, nrhs), dim3(S::threads), smem, s, a));
+    RTM_CUDA(launch_dependent(k_fast_x_mix_3<T, NP, SUB, MINB>, dim3((a.Q + S::teams - 1) / S::teams, SUB, nrhs), dim3(S::threads), smem, s, a));
     count_launch();
     return RTM_OK;
 }
@@ -983,7 +1029,7 @@ template <typename T, int NP> int launch_x(const GridArgs<T>& a, int nrhs, int k
     if constexpr (sizeof(T) == 8) {
         if (kind == kMixDirect3) return launch_x_direct<T, NP, 3>(a, nrhs, s);
     }
-    if constexpr (three_step(NP, sizeof(T) == 8)) return launch_x_3<T, NP>(a, nrhs, s);
+    if constexpr (three_step(NP, sizeof(T) == 8)) return launch_x_3<T, NP, 2>(a, nrhs, s);
     else return launch_x_direct<T, NP, 1>(a, nrhs, s);
 }
 
@@ -1015,6 +1061,29 @@ template <typename T> int dispatch_x(const GridArgs<T>& a, int nrhs, int kind, c
 }
 
 }  // namespace
+
+bool three_step_length(int n, bool fp64) { return n == 256 || n == 512 || (!fp64 && n == 1024); }
+
+namespace {
+template <typename T, int N> int three_step_of(int pass, const GridArgs<T>& a, int nrhs, const void* x, void* y, cudaStream_t s) {
+    if (pass == kRegXMix) return a.nsx == 2 ? launch_x_3<T, N, 2>(a, nrhs, s) : launch_x_3<T, N, 1>(a, nrhs, s);
+    return a.nsy == 2 ? launch_y_3<T, N, 2>(a, nrhs, x, y, pass == kRegYFwd, s)
+                      : launch_y_3<T, N, 1>(a, nrhs, x, y, pass == kRegYFwd, s);
+}
+}  // namespace
+
+template <typename T>
+int launch_three_step(int pass, const GridArgs<T>& a, int nrhs, const void* x, void* y, cudaStream_t s) {
+    switch (pass == kRegXMix ? a.P : a.Q) {
+        case 256: return three_step_of<T, 256>(pass, a, nrhs, x, y, s);
+        case 512: return three_step_of<T, 512>(pass, a, nrhs, x, y, s);
+        default:
+            if constexpr (sizeof(T) == 4) return three_step_of<T, 1024>(pass, a, nrhs, x, y, s);
+            return fail(RTM_ERR_UNSUPPORTED, "transform size");
+    }
+}
+template int launch_three_step<double>(int, const GridArgs<double>&, int, const void*, void*, cudaStream_t);
+template int launch_three_step<float>(int, const GridArgs<float>&, int, const void*, void*, cudaStream_t);
 
 bool fast_split_eligible(int P, int Q, bool fp64) {
     auto ok = [&](int n) { return n >= 32 && n <= (fp64 ? 512 : 1024) && (n & (n - 1)) == 0; };
