@@ -56,10 +56,10 @@ int BatchOp::apply(const void* x, void* y, int nrhs, cudaStream_t s, SkipFlags s
     if (fused) {
         if (work.bytes < plates[0]->work_bytes_per_rhs() * ops.size())
             return fail(RTM_ERR_ARG, "the plate batch was not reserved");
-        RTM_TRY(apply_plate_batch(plates, descs.ptr, stride, work.ptr, fault, x, y, s, skip));
+        return apply_plate_batch(plates, descs.ptr, stride, work.ptr, fault, x, y, s, skip);  // zeros the tails as well
     } else if (fused_bj) {
-        RTM_TRY(apply_block_jacobi_batch(descs.as<BjShape>(), (int)ops.size(), bj_blocks, bj_S, precision, x, y, stride,
-                                         s, skip));
+        return apply_block_jacobi_batch(descs.as<BjShape>(), (int)ops.size(), bj_blocks, bj_S, precision, x, y, stride,
+                                        s, skip);  // and so does this
     } else {
         const size_t elem = precision == RTM_FP64 ? sizeof(double2) : sizeof(float2);
         for (size_t k = 0; k < ops.size(); ++k) {

@@ -238,7 +238,8 @@ __global__ void k_bj_apply(const BjShape g, const T2* __restrict__ x, T2* __rest
     else bj_rows<T2, 0>(g, x + rhs * n, y + rhs * n, t);
 }
 
-// k_bj_apply for a batch of block-Jacobi operators: right-hand side k takes entry k's blocks.
+// k_bj_apply for a batch of block-Jacobi operators: right-hand side k takes entry k's blocks, and its vector is zero behind
+// the entry's rooftops.
 template <typename T2>
 __global__ void k_bj_apply_batch(const BjShape* __restrict__ entries, const T2* __restrict__ x, T2* __restrict__ y,
                                  int64_t stride, const int* skip, int skip_stride) {
@@ -247,6 +248,9 @@ __global__ void k_bj_apply_batch(const BjShape* __restrict__ entries, const T2* 
     if (skip && skip[(int64_t)rhs * skip_stride]) return;
     const BjShape e = entries[rhs];
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    for (int64_t i = (int64_t)(e.cx - 1) * e.cy + (int64_t)e.cx * (e.cy - 1) + t; i < stride;
+         i += (int64_t)gridDim.x * blockDim.x)
+        y[rhs * stride + i] = T2{};
     if (e.S == 8) bj_rows<T2, 8>(e, x + rhs * stride, y + rhs * stride, t);
     else bj_rows<T2, 0>(e, x + rhs * stride, y + rhs * stride, t);
 }
