@@ -14,6 +14,8 @@
 // the state of its right-hand side and does nothing once that solve is done; the host launches
 // `check_every` iterations, then reads the done flags once. Converged systems thus stop exactly at
 // the reference's iteration, and the extra launched iterations are no-ops.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -929,12 +931,14 @@ template <typename T2> static void launch_orth(const T2* V, T2* w, int64_t n, in
 // meet at two barriers; every CTA then sums the per-CTA partials itself, in one order. The norm needs no third one: the
 // last correction c is orthogonal to what it leaves, so ||w - V c||^2 = ||w||^2 - ||c||^2 with ||w||^2 summed beside c.
 // That loses nothing while c is small, as a second projection's is (rounding of the first); where ||c||^2 is above
-// kArnLeft of ||w||^2 (a second pass after heavy cancellation, or one pass alone) the norm is summed after all. A CTA keeps its chunk of w in shared memory from the first pass to the last, and as many of the basis
-// columns as fit beside it, so that these are read once instead of four times. One more CTA per right-hand side
-// holds no rows: it runs the rotations of the new Hessenberg column while the others subtract the last projection.
+// kArnLeft of ||w||^2 (a second pass after heavy cancellation, or one pass alone) the norm is summed after all.
+// A CTA keeps its chunk of w in shared memory from the first pass to the last, and as many of the basis columns as fit
+// beside it, so that these are read once instead of four times. One more CTA per right-hand side holds no rows: it runs
+// the rotations of the new Hessenberg column while the others subtract the last projection.
 //
-// Bound: the basis's L2 bandwidth and three barriers. 256 x 256 faces, one right-hand side, 100 iterations: the three
-// passes and k_gm_next took 46 us a step, four launches each waiting for the slowest CTA's chain of loads and sums.
+// Bound: the basis's L2 bandwidth and two barriers. 256 x 256 faces, one right-hand side, 100 iterations: the three
+// passes and k_gm_next took 46 us a step, four launches each waiting for the slowest CTA's chain of loads and sums; this
+// takes 35 to 37 (18 for the first column, 0.4 a column that stays in shared memory, 0.9 a column beyond).
 constexpr int kArnThreads = 512, kArnWarps = kArnThreads / 32, kArnCols = kStreamCols / kArnWarps;
 constexpr int kArnParts = 2 * kStreamCols + 2;  // partials a CTA
 constexpr int kArnoldiRows = 2048;
@@ -1400,6 +1404,208 @@ __global__ void k_gm_cycle_end(GmState* st, int nrhs) {
     st[rhs].skip_step = 1;
 }
 
+// --------------------------------------------------------------------------------------------
+// COCG's vector work of an iteration on up to kClusterRows rows in one launch a system, by a cluster of up to 8 CTAs that
+// keep their rows in registers and exchange the sums through shared memory. CTA `rank` takes the row chunks rank + C k,
+// k < K, so the chunks' sums and their total add as in the kernels above, to the last bit. Launches bound such solves, and
+// each of these kernels took 2 to 5 us for some 100 KB. 32 iterations without a preconditioner, whole solves: 32 x 32 faces
+// 931 -> 705 us (32 systems 1074 -> 850), 64 x 64 947 -> 762 (1542 -> 1295), 90 x 90 1245 -> 1136; with a circulant 1465 ->
+// 1184, 1559 -> 1316 and 1872 -> 1734. Four chunks a CTA pay only while the clusters fit the device in one wave (90 x 90, 32
+// systems: 2791 us in three launches, 3032 in this one); sums and iterates are the same either way.
+constexpr int kClusterMax = 8, kClusterChunks = 32;
+constexpr int64_t kClusterRows = (int64_t)kClusterChunks * kRowChunk;
+
+// Cluster size and chunks a CTA for n rows (none: the kernels above).
+struct CgCluster {
+    int ctas = 0, per = 0;
+    CgCluster(int64_t n, int nrhs) {
+        const int chunks = reduce_blocks(n);
+        if (n > kClusterRows || (chunks > 2 * kClusterMax && nrhs * kClusterMax > 148)) return;
+        ctas = 1;
+        while (ctas < chunks && ctas < kClusterMax) ctas *= 2;
+        per = 1;
+        while (per * ctas < chunks) per *= 2;
+    }
+};
+
+// The sums of the CTA's chunks, to slot rank + C k of every CTA of the cluster.
+template <int K>
+__device__ __forceinline__ void cluster_put(double2 (&acc)[K], double2* slots, const cooperative_groups::cluster_group& cl) {
+    __shared__ double2 both[K];
+    block_sum<K>(acc, both);
+    const int C = (int)cl.num_blocks(), t = threadIdx.x;
+    if (t < K * C) cl.map_shared_rank(slots, t / K)[(int)cl.block_rank() + C * (t % K)] = both[t % K];
+}
+
+// cta_total of the 32 slots, by every warp.
+__device__ __forceinline__ double2 slots_total(const double2* slots) {
+    double2 v = slots[threadIdx.x & 31];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        v.x += __shfl_down_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_down_sync(0xffffffffu, v.y, o);
+    }
+    return make_double2(__shfl_sync(0xffffffffu, v.x, 0), __shfl_sync(0xffffffffu, v.y, 0));
+}
+
+// k_cg_dq and k_cg_update; PLAIN (no preconditioner): the next iteration's k_cg_dir as well.
+template <typename T2, int K, bool PLAIN>
+__global__ void __launch_bounds__(kRT) k_cg_step(T2* __restrict__ x, T2* __restrict__ r, T2* __restrict__ d,
+                                                 const T2* __restrict__ q, int64_t n, CgState* st, double* hist,
+                                                 int hist_stride) {
+    __shared__ double2 slots[3][kClusterChunks];
+    griddep_wait();
+    const int rhs = blockIdx.y;
+    CgState& S = st[rhs];
+    if (S.done) return;
+    const double2 rho0 = S.rho;
+    const double bnorm = S.bnorm, tol = S.tol;
+    const int iteration = S.iteration + 1, most = S.max_iterations;
+    const auto cl = cooperative_groups::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    if (threadIdx.x < 3 * kClusterChunks) slots[threadIdx.x / kClusterChunks][threadIdx.x % kClusterChunks] = make_double2(0, 0);
+    cl.sync();  // every CTA has started, zeroed its slots and read the state
+    T2 dv[2 * K], qv[2 * K], rv[2 * K];
+    double2 dq[K];
+    const int64_t base = rhs * n;
+    auto row = [&](int k, int h) { return (int64_t)(rank + C * k) * kRowChunk + h * kRT + threadIdx.x; };
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        dq[k] = make_double2(0, 0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t i = row(k, h);
+            if (i < n) {
+                dv[2 * k + h] = d[base + i];
+                qv[2 * k + h] = q[base + i];
+                rv[2 * k + h] = r[base + i];
+                dq[k] = dadd(dq[k], dmul(to_d2(dv[2 * k + h]), to_d2(qv[2 * k + h])));
+            }
+        }
+    }
+    cluster_put<K>(dq, slots[0], cl);
+    cl.sync();
+    const double2 alpha = ddiv(rho0, slots_total(slots[0]));
+    double2 norm[K], rr[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        norm[k] = rr[k] = make_double2(0, 0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t i = row(k, h);
+            if (i < n) {
+                const double2 xv = dadd(to_d2(x[base + i]), dmul(alpha, to_d2(dv[2 * k + h])));
+                const double2 aq = dmul(alpha, to_d2(qv[2 * k + h]));
+                const double2 rv0 = to_d2(rv[2 * k + h]);
+                const T2 rs = from_d2<T2>(make_double2(rv0.x - aq.x, rv0.y - aq.y));
+                x[base + i] = from_d2<T2>(xv);
+                r[base + i] = rs;
+                rv[2 * k + h] = rs;
+                const double2 rd = to_d2(rs);
+                norm[k].x += rd.x * rd.x + rd.y * rd.y;
+                if (PLAIN) rr[k] = dadd(rr[k], dmul(rd, rd));
+            }
+        }
+    }
+    cluster_put<K>(norm, slots[1], cl);
+    if (PLAIN) cluster_put<K>(rr, slots[2], cl);
+    cl.sync();
+    const double h = sqrt(slots_total(slots[1]).x) / bnorm;
+    const double2 rho = PLAIN ? slots_total(slots[2]) : rho0;
+    const double2 beta = ddiv(rho, rho0);
+    const bool converged = h < tol;
+    // A breakdown (d^T A d = 0) leaves Inf or NaN (ConjugateGradient.m:55-58).
+    const bool done = converged || !isfinite(h) || iteration >= most;
+    if (rank == 0 && threadIdx.x == 0) {
+        if (PLAIN) {
+            S.beta = beta;
+            S.rho = rho;
+        }
+        S.iteration = iteration;
+        hist[(int64_t)rhs * hist_stride + iteration] = h;
+        S.converged = converged;
+        S.done = done;
+    }
+    if (!PLAIN || done) return;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int h2 = 0; h2 < 2; ++h2) {
+            const int64_t i = row(k, h2);
+            if (i < n) d[base + i] = from_d2<T2>(dadd(to_d2(rv[2 * k + h2]), dmul(beta, to_d2(dv[2 * k + h2]))));
+        }
+}
+
+// k_cg_rz and k_cg_dir.
+template <typename T2, int K>
+__global__ void __launch_bounds__(kRT) k_cg_rz_dir(const T2* __restrict__ r, const T2* __restrict__ z, T2* __restrict__ d,
+                                                   int64_t n, CgState* st) {
+    __shared__ double2 slots[kClusterChunks];
+    griddep_wait();
+    const int rhs = blockIdx.y;
+    CgState& S = st[rhs];
+    if (S.done) return;
+    const double2 rho0 = S.rho;
+    const bool first = S.iteration == 0;
+    const auto cl = cooperative_groups::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    if (threadIdx.x < kClusterChunks) slots[threadIdx.x] = make_double2(0, 0);
+    cl.sync();  // every CTA has started, zeroed its slots and read the state
+    T2 zv[2 * K];
+    double2 rz[K];
+    const int64_t base = rhs * n;
+    auto row = [&](int k, int h) { return (int64_t)(rank + C * k) * kRowChunk + h * kRT + threadIdx.x; };
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        rz[k] = make_double2(0, 0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t i = row(k, h);
+            if (i < n) {
+                zv[2 * k + h] = z[base + i];
+                rz[k] = dadd(rz[k], dmul(to_d2(r[base + i]), to_d2(zv[2 * k + h])));
+            }
+        }
+    }
+    cluster_put<K>(rz, slots, cl);
+    cl.sync();
+    const double2 rho = slots_total(slots);
+    const double2 beta = first ? make_double2(0, 0) : ddiv(rho, rho0);
+    if (rank == 0 && threadIdx.x == 0) {
+        S.beta = beta;
+        S.rho = rho;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int64_t i = row(k, h);
+            if (i < n)
+                d[base + i] = first ? zv[2 * k + h]
+                                    : from_d2<T2>(dadd(to_d2(zv[2 * k + h]), dmul(beta, to_d2(d[base + i]))));
+        }
+}
+
+template <typename T2>
+static cudaError_t launch_cg_step(const CgCluster& c, bool plain, T2* x, T2* r, T2* d, const T2* q, int64_t n, int nrhs,
+                                  CgState* st, double* hist, int hs, cudaStream_t s) {
+    auto go = [&](auto kernel) {
+        return launch_dependent_clusters(kernel, c.ctas, dim3(c.ctas, nrhs), dim3(kRT), s, x, r, d, q, n, st, hist, hs);
+    };
+    if (c.per == 1) return plain ? go(k_cg_step<T2, 1, true>) : go(k_cg_step<T2, 1, false>);
+    if (c.per == 2) return plain ? go(k_cg_step<T2, 2, true>) : go(k_cg_step<T2, 2, false>);
+    return plain ? go(k_cg_step<T2, 4, true>) : go(k_cg_step<T2, 4, false>);
+}
+
+template <typename T2>
+static cudaError_t launch_cg_rz_dir(const CgCluster& c, const T2* r, const T2* z, T2* d, int64_t n, int nrhs, CgState* st,
+                                    cudaStream_t s) {
+    auto go = [&](auto kernel) {
+        return launch_dependent_clusters(kernel, c.ctas, dim3(c.ctas, nrhs), dim3(kRT), s, r, z, d, n, st);
+    };
+    return c.per == 1 ? go(k_cg_rz_dir<T2, 1>) : c.per == 2 ? go(k_cg_rz_dir<T2, 2>) : go(k_cg_rz_dir<T2, 4>);
+}
+
 // ============================================================================================
 // Shared helpers
 // out = b - t where flag (stride) is zero.
@@ -1585,9 +1791,26 @@ static int cocg(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* bv
     std::vector<CgState> host(nrhs);
     int launched = 0;
     res.matvecs = x0 ? 1 : 0;
+    const CgCluster cluster(n, nrhs);
+    if (cluster.ctas && !M) {  // the first direction; k_cg_step leaves the next ones
+        RTM_CUDA(launch_dependent(k_cg_dir<T2>, grid, dim3(kRT), 0, s, (const T2*)zp, d.as<T2>(), n, (const CgState*)st));
+        count_launch();
+    }
     // `every` iterations as one graph; iterations past the stopping test are no-ops on the device.
     auto chunk_body = [&]() -> int {
         for (int it = 0; it < every; ++it) {
+            if (cluster.ctas) {
+                if (M) {
+                    RTM_TRY(M->apply(r.ptr, z.ptr, nrhs, s, skip));
+                    RTM_CUDA(launch_cg_rz_dir<T2>(cluster, r.as<T2>(), z.as<T2>(), d.as<T2>(), n, nrhs, st, s));
+                    count_launch();
+                }
+                RTM_TRY(A->apply(d.ptr, q.ptr, nrhs, s, skip));
+                RTM_CUDA(launch_cg_step<T2>(cluster, !M, x, r.as<T2>(), d.as<T2>(), q.as<T2>(), n, nrhs, st,
+                                            hist.as<double>(), hs, s));
+                count_launch();
+                continue;
+            }
             if (M) {
                 RTM_TRY(M->apply(r.ptr, z.ptr, nrhs, s, skip));
                 RTM_CUDA(launch_dependent(k_cg_rz<T2>, grid, dim3(kRT), 0, s, (const T2*)r.as<T2>(), (const T2*)zp, n, st,

@@ -209,3 +209,64 @@ def test_assembled_generators(grid, sizes, orders):
     for g, w in zip(got, (want.magnetic_xx, want.magnetic_yy, want.electric)):
         if w is not None and w.size:
             assert rel(g, w) < 1e-12
+
+
+@pytest.mark.parametrize("grid", [(256, 33), (33, 256), (255, 35), (512, 21), (19, 511), (256, 256), (1024, 18), (17, 1023)])
+@pytest.mark.parametrize("precision", ["double", "single"])
+def test_lines_of_three_steps(grid, precision):
+    """Transform lengths 256, 512 and 1024 along either direction or both, beside lengths of the register-resident form
+    and an odd number of lines; a last row of padding; one vector and three. The split product, the circulant, and the
+    embedding whose period 2 n - 2 is 256."""
+    from oracle import preconditioner as Q, spectra as S
+
+    R, prob, rt, gen = _setup(*grid)
+    v = random_vector(3 * rt.count, seed=9)
+    sub = S.subband_spectra(gen, rt.size_x, rt.size_y)
+    circ = Q.circulant(gen, rt.size_x, rt.size_y, kernel="rChan")
+    op, pc = R.Operator(prob, precision=precision, maxRhs=3), R.Preconditioner(prob, kernel="rChan", precision=precision)
+    got, pre = op.apply(v, nrhs=3), pc.apply(v, nrhs=3)
+    for k in range(3):
+        part = slice(k * rt.count, (k + 1) * rt.count)
+        assert rel(got[part], S.split_apply(rt, sub, rt.content, v[part])) < (1e-13 if precision == "double" else 2e-5)
+        assert rel(pre[part], S.fft_apply(rt, circ, rt.content, v[part])) < (1e-11 if precision == "double" else 2e-5)
+    assert rel(op.apply(v[:rt.count]), got[:rt.count]) < 1e-15
+    if grid == (33, 256):
+        R, prob, rt, gen = _setup(129, grid[0])
+        emb = S.embedding_spectra(gen, rt.size_x, rt.size_y)
+        got = R.Operator(prob, product="fft", precision=precision).apply(v[:rt.count])
+        assert rel(got, S.fft_apply(rt, emb, rt.content, v[:rt.count])) < (1e-13 if precision == "double" else 2e-5)
+
+
+@pytest.mark.parametrize("grid", [(2, 2), (16, 17), (16, 18), (23, 23), (45, 46), (46, 46), (64, 65), (65, 65), (91, 91),
+                                  (91, 92)])
+@pytest.mark.parametrize("preconditioned", [True, False])
+def test_cocg_steps_by_row_chunks(grid, preconditioned):
+    """One chunk of rows to one more than a cluster takes, and the first size above: the residuals of five iterations,
+    which rounding has not yet moved, for two systems and a zero one, and the current they leave."""
+    import numpy as np
+
+    from oracle import preconditioner as Q, solvers, spectra as S
+
+    R, prob, rt, gen = _setup(*grid)
+    sub = S.subband_spectra(gen, rt.size_x, rt.size_y)
+    A = lambda v: S.split_apply(rt, sub, rt.content, v)  # noqa: E731
+    pc = M = None
+    if preconditioned:
+        pc = R.Preconditioner(prob, kernel="rChan")
+        spec = Q.circulant(gen, rt.size_x, rt.size_y, kernel="rChan")
+        M = lambda v: S.fft_apply(rt, spec, rt.content, v)  # noqa: E731
+    n = rt.count
+    limit = min(5, n)
+    b = np.concatenate([random_vector(n, seed=3), np.zeros(n), random_vector(n, seed=4)])
+    got = R.Solver("cg", tolerance=1e-14, maxIterationCount=limit).solve(R.Operator(prob, maxRhs=3), b, preconditioner=pc,
+                                                                       nrhs=3)
+    for k, r in enumerate(got):
+        if k == 1:
+            assert r.converged() and r.iterationCount() == 0 and not np.any(r.solution())
+            continue
+        want = solvers.solve("cg", A, b[k * n:(k + 1) * n], tol=1e-14, maxit=limit, precond=M)
+        count = min(r.iterationCount(), want.iteration_count) + 1
+        above = want.residual_norms[:count] > 1e-10  # the smallest system converges within the limit
+        assert above[0] and np.allclose(r.residualNorms()[:count][above], want.residual_norms[:count][above], rtol=1e-9)
+        true = np.linalg.norm(b[k * n:(k + 1) * n] - A(r.solution())) / np.linalg.norm(b[k * n:(k + 1) * n])
+        assert abs(true - r.residualNorm()) < 1e-10
