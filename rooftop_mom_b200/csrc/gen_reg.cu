@@ -3,7 +3,8 @@
 // The generators' embeddings and circulant folds are even in both directions. Along x the unmodulated source at P - i is
 // the one at i, negated for the odd subband, so the y pass transforms P / 2 + 1 columns; along y the transforms are even
 // in the frequency, so Q / 2 + 1 rows are kept, transformed along x and written twice. Twelve spectra of 256 x 256 points:
-// 88 + 42 us on the Stockham kernels of grid.cu (255 registers, 11 % of the warps active), which write and read every row.
+// 88 + 42 us on the Stockham kernels of grid.cu (255 registers, 11 % of the warps active), which write and read every row; 33 + 8
+// here.
 #include <algorithm>
 
 #include "gen.cuh"

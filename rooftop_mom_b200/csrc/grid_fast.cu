@@ -446,12 +446,15 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
     }
 }
 
-// The x lines that run in three steps, a thread holding both components: they share the twiddles, the phases and E, and
-// meet in registers, and the small radices need half the registers. The L1 pipe bounds both forms (FP64 512 x 512 with
-// four vectors: 49 % busy at 8 warps an SM before, 70 % now). Product, two steps -> three: FP64 256 x 256 15.9 -> 14.2 us,
-// four vectors 42.9 -> 38.3; 512 x 512 46.6 -> 37.2 and 185 -> 152; FP32 512 x 512 29.6 -> 27.9 and 94 -> 81; 1024 x 1024
-// 104 -> 93 and 382 -> 350. FP32 256 x 256 stays on two steps (12.4 against 12.5 us, 23.4 against 24.9): its lines exchange
-// within their warps there; shorter lines leave too few threads for three steps.
+// The lengths of split products that run in three steps, a thread holding both components of an x line (they share the
+// twiddles, the phases and E, and meet in registers) or both subbands of a column; the small radices need half the
+// registers. The L1 pipe bounds both forms of the x-mix (FP64 512 x 512 with four vectors: 49 % busy at 8 warps an SM
+// before, 70 % now). Product, two steps -> three, one vector and four: FP64 256 x 256 15.9 -> 13.5 us and 42.9 -> 36.8; 512
+// x 512 46.6 -> 37.2 and 185 -> 139; FP32 512 x 512 29.6 -> 25.2 and 94 -> 81; 1024 x 1024 104 -> 89 and 382 -> 345. FP32
+// 256 x 256 stays on two steps (x-mix in three: 12.5 against 12.4 us, 24.9 against 23.4): its lines exchange within their
+// warps there; shorter lines leave too few threads for three steps. Without subbands every such length gains, FP32 256 too
+// (circulants, against the register-resident lines of grid_reg.cu: FP64 256 x 256 20.5 -> 11.3, 512 x 512 35.2 -> 17.3;
+// FP32 17.9 -> 10.1, 27.9 -> 15.4, 1024 x 1024 110 -> 36).
 constexpr bool three_step(int n, bool fp64) { return fp64 ? n == 256 || n == 512 : n == 512 || n == 1024; }
 
 // SUB: the subbands along x (2: a split product, 1: an embedding or a circulant).
@@ -945,6 +948,8 @@ template <typename T, int NQ, int SUB> int launch_y_3(const GridArgs<T>& a, int 
                                              cudaStream_t s) {
     using T2 = typename Cx<T>::T2;
     using S = Y3<T, NQ>;
+    // CTAs an SM; with TI columns of 64 bytes (FP64 512 x 512 with four vectors: 139 us; 2 columns and 3 CTAs 150, one
+    // CTA 155; FP32 1024 x 1024: 345, 4 columns and 2 CTAs 352).
     constexpr int MINB = sizeof(T) == 8 ? (NQ == 256 ? 3 : 2) : (NQ == 1024 ? 1 : 2);
     static DeviceOnce once;
     RTM_TRY(once([]() -> int {

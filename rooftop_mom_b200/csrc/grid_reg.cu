@@ -3,7 +3,9 @@
 //
 // The same three passes as k_grid_y_fwd / k_grid_x_mix / k_grid_y_inv in grid.cu (the reference's
 // @SplitFFTApplicator/applyBothDirections_.m:14-85, FFTApplicator.m:52-87), whose Stockham stages keep 255
-// registers a thread and one CTA an SM (8 % of the warps active) and pass every radix through shared memory.
+// registers a thread and one CTA an SM (8 % of the warps active) and pass every radix through shared memory. An FP64 product
+// of 301 x 187 faces: 175 us a call there, 45 here; both wait for loads and exchanges with few warps in flight, not for
+// bandwidth or arithmetic. Passes along lengths of 256, 512 and 1024 run in three steps (grid_fast.cu).
 #include <algorithm>
 
 #include "grid.h"

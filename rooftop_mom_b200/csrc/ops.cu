@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(kBuildThreads) k_bj_build(const BjShape g, con
 // the warp (blocks of 1, 2, 4, 8 or 16 unknowns, 2 x 2 faces among them), the S threads of a block each gather
 // their own x(idx_r) and pass it to the others by warp shuffles, so a thread issues one vector load instead of S;
 // the sum runs over c in the same order either way. Bound: the vectors (read and written once); the inverses
-// stay in L1. The 256 x 256 plate, FP64: 7.2 us with an inverse and an index list per block.
+// stay in L1. The 256 x 256 plate, FP64: 7.2 us with an inverse and an index list per block, 5.4 with a
+// class's (cold caches; 3.1 warm).
 template <typename T2, int SC>  // SC: S as a compile-time constant (the loops unroll), or 0
 __device__ __forceinline__ void bj_rows(const BjShape& g, const T2* __restrict__ xr, T2* __restrict__ yr, int64_t t) {
     const int S = SC ? SC : g.S;
