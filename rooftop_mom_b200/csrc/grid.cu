@@ -462,9 +462,9 @@ static int apply_t(const GridApplicator& g, const void* xv, void* yv, int nrhs, 
 }
 
 int GridApplicator::reserve(int nrhs) {
-    // kernel attributes and the fault word are set up here, outside of any stream capture
+    // the Stockham kernels' attributes are set up here; the register-resident and power-of-two ones set theirs at their
+    // first launch, which a stream capture allows
     RTM_TRY(precision == RTM_FP64 ? set_smem_attrs<double>() : set_smem_attrs<float>());
-    RTM_TRY(device_fault_word(&fault));
     if (nrhs <= max_rhs && (mode == kStrip || work.bytes >= work_bytes_per_rhs() * (size_t)nrhs)) return RTM_OK;
     if (mode != kStrip) RTM_TRY(work.alloc(work_bytes_per_rhs() * (size_t)nrhs));
     max_rhs = std::max(max_rhs, nrhs);
@@ -535,7 +535,6 @@ int apply_plate_batch(const std::vector<const GridApplicator*>& plates, const vo
 
 int GridApplicator::apply(const void* x, void* y, int nrhs, cudaStream_t s, SkipFlags skip) {
     if (nrhs < 1 || nrhs > max_rhs) return fail(RTM_ERR_ARG, "more right-hand sides than the product reserved");
-    if (!fault) RTM_TRY(device_fault_word(&fault));
     return precision == RTM_FP64 ? apply_t<double>(*this, x, y, nrhs, s, skip, work.ptr, fault)
                                  : apply_t<float>(*this, x, y, nrhs, s, skip, work.ptr, fault);
 }
@@ -557,10 +556,8 @@ int apply_fixed_scratch(const GridApplicator& g, const void* x, void* y, int nrh
                                       std::to_string(cap) + " bytes");
     void* work = nullptr;
     if (g.mode != kStrip) RTM_TRY(fixed_scratch_address(&work));
-    int* fault = nullptr;
-    RTM_TRY(device_fault_word(&fault));
-    return g.precision == RTM_FP64 ? apply_t<double>(g, x, y, nrhs, s, SkipFlags{}, work, fault)
-                                   : apply_t<float>(g, x, y, nrhs, s, SkipFlags{}, work, fault);
+    return g.precision == RTM_FP64 ? apply_t<double>(g, x, y, nrhs, s, SkipFlags{}, work, g.fault)
+                                   : apply_t<float>(g, x, y, nrhs, s, SkipFlags{}, work, g.fault);
 }
 
 // ============================================================================================
@@ -744,6 +741,7 @@ int build_product(const DeviceGenerators& g, double size_x, double size_y, int p
     out.max_rhs = std::max(1, max_rhs);
     out.lean = product == RTM_PRODUCT_LEAN;
     if (out.content == RTM_NONE) return fail(RTM_ERR_ARG, "a single face carries no rooftop");
+    RTM_TRY(device_fault_word(&out.fault));  // may allocate pinned memory: here, as a first apply may run under capture
     GenArgs a{};
     a.kind = kSrcEmbed;
     if (product == RTM_PRODUCT_FFT) {
@@ -1181,6 +1179,7 @@ int build_circulant(const DeviceGenerators& g, double size_x, double size_y, int
     out.size_x = size_x;
     out.size_y = size_y;
     out.max_rhs = 1;
+    RTM_TRY(device_fault_word(&out.fault));
     out.P = cx;
     out.Q = cy;
     out.nsx = out.nsy = 1;

@@ -56,7 +56,7 @@ struct GridApplicator : LinearOp {
     DeviceBuffer spec;      // GEN3: [sub][3][Q][P]; BLOCK4: [4][Q][P]; STRIP: [sub][P]
     DeviceBuffer work;      // W
     int spec_blocks = 0;    // blocks stored
-    int* fault = nullptr;   // the device's fault word (looked up in reserve(), outside any capture)
+    int* fault = nullptr;   // the device's fault word, looked up when the product is built: a first apply may run under capture
     FastSchedule sched;     // schedule of the power-of-two kernels (set when the product is built)
 
     // y = A x on the device for nrhs vectors of length n (precision of the product).
