@@ -301,6 +301,7 @@ struct GmState {
     int skip_update;  // = !cycle_ran: the preconditioner's skip flag for the right-preconditioned update
     unsigned int counter;
     unsigned int bar, bar_base;  // k_gm_arnoldi: its barrier's arrivals, and their count before this step
+    int timed_out;    // a CTA of k_gm_arnoldi gave up waiting at its barrier: the solve fails
 };
 
 struct GmArrays {
@@ -944,7 +945,6 @@ constexpr int kArnParts = 2 * kStreamCols + 2;  // partials a CTA
 constexpr int kArnoldiRows = 2048;
 constexpr size_t kArnSmem = 216 * 1024;  // dynamic shared memory (about 7 KB more are static)
 constexpr double kArnLeft = 1e-6;  // the subtraction's relative error then stays below 1e-6 of its terms' rounding
-constexpr unsigned kArnPolls = 1u << 21;  // of a barrier, about 0.7 us each
 
 __device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
     unsigned v;
@@ -952,21 +952,21 @@ __device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
     return v;
 }
 
-// Waits until `target` arrivals (modulo 2^32) have been counted; false, with the fault word set, when they have not
-// within kArnPolls polls.
-__device__ __forceinline__ bool arnoldi_barrier(unsigned* bar, unsigned target, int* fault) {
+// Waits until `target` arrivals (modulo 2^32) have been counted; false, with the state's flag set, when they have not
+// within `polls` polls of about 0.7 us.
+__device__ __forceinline__ bool arnoldi_barrier(GmState& S, unsigned target, unsigned polls) {
     __shared__ int met;
     __syncthreads();
     if (threadIdx.x == 0) {
         // release and acquire at the device's scope order what the CTA wrote before and reads after
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(bar) : "memory");
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(&S.bar) : "memory");
         met = 0;
-        for (unsigned i = 0; i < kArnPolls; ++i)
-            if ((int)(load_acquire(bar) - target) >= 0) {
+        for (unsigned i = 0; i < polls; ++i)
+            if ((int)(load_acquire(&S.bar) - target) >= 0) {
                 met = 1;
                 break;
             }
-        if (!met && fault) *static_cast<volatile int*>(fault) = (int)RTM_ERR_TIMEOUT;
+        if (!met) atomicExch(&S.timed_out, 1);
     }
     __syncthreads();
     return met != 0;
@@ -1011,10 +1011,12 @@ __device__ __forceinline__ void arnoldi_dots(const T2* __restrict__ V, int64_t c
 }
 
 // V: the basis [m + 1][nrhs][n], read up to column `step` and written at column step + 1 (vnext: the same memory).
+// Any CTA may be the one that gives up at a barrier, with others past it: every one that does sets timed_out, the later
+// steps of the right-hand side do nothing, and the host returns RTM_ERR_TIMEOUT from the state it reads after each cycle.
 template <typename T2>
 __global__ void __launch_bounds__(kArnThreads, 1)
     k_gm_arnoldi(const T2* __restrict__ V, T2* vnext, const T2* __restrict__ w, int64_t n, int nrhs, GmState* st, GmArrays ar,
-                 double2* parts, int passes, int chunk, int room, int* fault) {
+                 double2* parts, int passes, int chunk, int room, unsigned polls) {
     using A2 = typename OrthAcc<T2>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double2 sum_h[kStreamCols], sum_c[kStreamCols], red[kStreamCols];
@@ -1023,7 +1025,10 @@ __global__ void __launch_bounds__(kArnThreads, 1)
     __shared__ double total;
     const int rhs = blockIdx.y, B = gridDim.x - 1, blk = blockIdx.x;
     GmState& S = st[rhs];
-    if (!S.active) return;
+    // timed_out may change under a CTA that starts late, so one thread reads it for all; the other fields change only
+    // behind the last barrier
+    const bool off = !S.active;
+    if (__syncthreads_or(threadIdx.x == 0 && *static_cast<volatile int*>(&S.timed_out)) || off) return;
     const int j = S.step, cols = j + 1, m = ar.m;
     const unsigned base = S.bar_base, all = gridDim.x;
     const bool scalar = blk == B;
@@ -1151,7 +1156,7 @@ __global__ void __launch_bounds__(kArnThreads, 1)
     __syncthreads();
     if (!scalar) dots(0);
     unsigned at = base + all;
-    bool met = arnoldi_barrier(&S.bar, at, fault);
+    bool met = arnoldi_barrier(S, at, polls);
     if (met) {
         gather(0, sum_h);
         if (passes == 2) {
@@ -1160,7 +1165,7 @@ __global__ void __launch_bounds__(kArnThreads, 1)
                 dots(1);
             }
             at += all;
-            met = arnoldi_barrier(&S.bar, at, fault);
+            met = arnoldi_barrier(S, at, polls);
             if (met) {
                 gather(1, sum_c);
                 gather_norm(0);
@@ -1200,22 +1205,14 @@ __global__ void __launch_bounds__(kArnThreads, 1)
         }
         if (again) {
             at += all;
-            met = arnoldi_barrier(&S.bar, at, fault);
+            met = arnoldi_barrier(S, at, polls);
             if (met) {
                 gather_norm(1);
                 sub2 = total;
             }
         }
     }
-    if (!met) {
-        // a barrier ran out: this right-hand side stops (the host reports the fault word)
-        if (scalar && tid == 0) {
-            S.active = 0;
-            S.skip_step = 1;
-            S.done = 1;
-        }
-        return;
-    }
+    if (!met) return;
     if (!scalar) {
         const double sub = sqrt(sub2), inv = sub != 0 ? 1.0 / sub : 0.0;
         T2* out = vnext + ((int64_t)(j + 1) * nrhs + rhs) * n + c0;
@@ -1265,7 +1262,7 @@ template <typename T2> static bool arnoldi_shape(int64_t n, int nrhs, int m, Arn
 
 template <typename T2>
 static int launch_arnoldi(const ArnoldiShape& a, T2* V, const T2* w, int64_t n, int nrhs, GmState* st, const GmArrays& ar,
-                          double2* parts, int passes, int* fault, cudaStream_t s) {
+                          double2* parts, int passes, unsigned polls, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.blocks + 1, nrhs);
     cfg.blockDim = dim3(kArnThreads);
@@ -1277,7 +1274,7 @@ static int launch_arnoldi(const ArnoldiShape& a, T2* V, const T2* w, int64_t n, 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     RTM_CUDA(cudaLaunchKernelEx(&cfg, k_gm_arnoldi<T2>, (const T2*)V, V, w, n, nrhs, st, ar, parts, passes, a.chunk, a.room,
-                                fault));
+                                polls));
     count_launch();
     return RTM_OK;
 }
@@ -1955,9 +1952,7 @@ static int gmres(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b
     DeviceBuffer parts;
     StreamSyncGuard parts_guard(s);
     const bool fused = arnoldi_shape<T2>(n, nrhs, m, &shape);
-    int* fault = nullptr;
     if (fused) {
-        RTM_TRY(device_fault_word(&fault));
         RTM_TRY(parts.alloc(sizeof(double2) * kArnParts * (size_t)shape.blocks * nrhs));
         RTM_CUDA(cudaFuncSetAttribute(k_gm_arnoldi<T2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kArnSmem));
     }
@@ -1989,7 +1984,7 @@ static int gmres(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b
             }
             if (fused) {
                 RTM_TRY(launch_arnoldi<T2>(shape, Vp, w.as<T2>(), n, nrhs, st, ar, parts.as<double2>(),
-                                           cfg.gram_schmidt_passes == 1 ? 1 : 2, fault, s));
+                                           cfg.gram_schmidt_passes == 1 ? 1 : 2, cfg.barrier_polls, s));
                 continue;
             }
             // CGS2: project (mode 0), subtract and project again (1), subtract the correction and take the
@@ -2030,7 +2025,11 @@ static int gmres(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b
         RTM_CUDA(cudaMemcpyAsync(host.data(), stb.ptr, sizeof(GmState) * nrhs, cudaMemcpyDeviceToHost, s));
         RTM_CUDA(cudaStreamSynchronize(s));
         bool all = true;
-        for (auto& hh : host) all = all && hh.done;
+        for (auto& hh : host) {
+            if (hh.timed_out)
+                return fail(RTM_ERR_TIMEOUT, "a barrier of an Arnoldi step ran out on the device; the solve has no result");
+            all = all && hh.done;
+        }
         if (all || cycles > cfg.max_iterations || (cfg.cancel && *cfg.cancel)) break;
         RTM_TRY(graph.run(s, cycle_body));
         ++cycles;
@@ -2195,6 +2194,7 @@ int solve_mixed(LinearOp* A64, LinearOp* A32, LinearOp* M32, const SolveConfig& 
         ic.right_preconditioned = 1;
         ic.gram_schmidt_passes = cfg.inner_gram_schmidt_passes;
         ic.cancel = cfg.cancel;
+        ic.barrier_polls = cfg.barrier_polls;
         SolveResult ir;
         if (inner_cg) RTM_TRY(cocg<float>(A32, M32, ic, r32.ptr, nullptr, d32.ptr, n, nrhs, ir, s));
         else RTM_TRY(gmres<float>(A32, M32, ic, r32.ptr, nullptr, d32.ptr, n, nrhs, ir, s));

@@ -23,6 +23,7 @@ struct SolveConfig {
     int gram_schmidt_passes = 2;   // GMRES: classical Gram-Schmidt passes per Arnoldi step (2: CGS2, or 1)
     int inner_gram_schmidt_passes = 1;  // mixed: the passes of the FP32 inner solves
     const std::atomic<int>* cancel = nullptr;  // nonzero: stop at the next host check (unconverged result)
+    unsigned barrier_polls = 1u << 21;  // GMRES: polls of a device-side barrier before the solve fails (1.5 s)
 };
 
 struct SolveResult {
