@@ -39,11 +39,10 @@ int zero_tails(void* y, int precision, int64_t stride, const int64_t* counts_dev
 
 int BatchOp::reserve(int nrhs) {
     if (nrhs != (int)ops.size()) return fail(RTM_ERR_ARG, "a plate batch applies to one vector per entry");
-    RTM_TRY(device_fault_word(&fault));
     if (fused) {
         const size_t need = plates[0]->work_bytes_per_rhs() * ops.size();
         if (work.bytes < need) RTM_TRY(work.alloc(need));
-        // the entries' own reserve sets up the kernels' attributes and their fault word
+        // the entries' own reserve sets up the kernels' attributes
         for (LinearOp* op : ops) RTM_TRY(op->reserve(1));
         return RTM_OK;
     }
@@ -56,7 +55,7 @@ int BatchOp::apply(const void* x, void* y, int nrhs, cudaStream_t s, SkipFlags s
     if (fused) {
         if (work.bytes < plates[0]->work_bytes_per_rhs() * ops.size())
             return fail(RTM_ERR_ARG, "the plate batch was not reserved");
-        return apply_plate_batch(plates, descs.ptr, stride, work.ptr, fault, x, y, s, skip);  // zeros the tails as well
+        return apply_plate_batch(plates, descs.ptr, stride, work.ptr, fault.ptr, x, y, s, skip);  // zeros the tails as well
     } else if (fused_bj) {
         return apply_block_jacobi_batch(descs.as<BjShape>(), (int)ops.size(), bj_blocks, bj_S, precision, x, y, stride,
                                         s, skip);  // and so does this
@@ -108,6 +107,7 @@ std::unique_ptr<BatchOp> make_batch(const std::vector<LinearOp*>& ops, int64_t s
             if (ok) b->plates.push_back(g);
         }
         if (ok) {
+            if ((*status = b->fault.acquire()) != RTM_OK) return nullptr;
             if ((*status = plate_descs(b->plates, b->descs, s)) != RTM_OK) return nullptr;
             b->fused = true;
         } else {

@@ -27,11 +27,16 @@ struct BatchOp : LinearOp {
     bool fused_bj = false;               // fused block-Jacobi preconditioners
     int bj_blocks = 0, bj_S = 0;         // fused block-Jacobi: the most blocks of an entry, their packed size
     DeviceBuffer descs, tails, work;     // fused: plate or block-Jacobi table, per-entry unknowns (device), W
-    int* fault = nullptr;
+    FaultWord fault;                     // fused products: the batch's kernels run for all entries
 
     int apply(const void* x, void* y, int nrhs, cudaStream_t s, SkipFlags skip) override;
     int reserve(int nrhs) override;
     double working_bytes() const override { return (double)work.bytes; }
+    bool take_fault() override {
+        bool any = fault.take();
+        for (LinearOp* op : ops) any |= op->take_fault();
+        return any;
+    }
 };
 
 // A batch over the given per-entry operators (all of one precision, each of n_k <= stride unknowns).

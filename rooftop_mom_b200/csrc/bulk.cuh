@@ -9,7 +9,7 @@
 // A wait gives up after kBulkWaitTries polls (each poll may suspend the thread for a short, hardware
 // chosen time; the bound is far above any real copy time). It then records RTM_ERR_TIMEOUT in the
 // fault word passed to it, and the caller returns without using the data; the host reads the word
-// after its next synchronisation (device_fault_check) and reports the timeout instead of a result.
+// after its next synchronisation (fault_check) and reports the timeout instead of a result.
 #pragma once
 
 #include <stdint.h>

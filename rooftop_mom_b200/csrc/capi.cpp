@@ -360,7 +360,7 @@ int rtm_operator_apply(rtm_operator* op, const void* x, void* y, int64_t n, int 
     RTM_TRY(out_prepare(y, n * nrhs, prec, where, o, s));
     RTM_TRY(op->op->apply(in.ptr, o.ptr, nrhs, s, SkipFlags{}));
     RTM_TRY(out_finish(y, n * nrhs, prec, where, o, s));
-    if (where == RTM_HOST || !stream) RTM_TRY(device_fault_check(s));
+    if (where == RTM_HOST || !stream) RTM_TRY(fault_check(s, {op->op.get()}));
     return RTM_OK;
 }
 
@@ -372,7 +372,7 @@ int rtm_operator_apply_fixed_scratch(const rtm_operator* op, const void* x, void
     RTM_TRY(check_rhs(nrhs));
     cudaStream_t s = pick(stream, op->stream);
     RTM_TRY(apply_fixed_scratch(*op->grid, x, y, nrhs, s));
-    if (!stream) RTM_TRY(device_fault_check(s));
+    if (!stream) RTM_TRY(fault_check(s, {op->op.get()}));
     return RTM_OK;
 }
 
@@ -466,7 +466,7 @@ int rtm_preconditioner_apply(rtm_preconditioner* pc, const void* x, void* y, int
     RTM_TRY(out_prepare(y, n * nrhs, prec, where, o, s));
     RTM_TRY(pc->op->apply(in.ptr, o.ptr, nrhs, s, SkipFlags{}));
     RTM_TRY(out_finish(y, n * nrhs, prec, where, o, s));
-    if (where == RTM_HOST || !stream) RTM_TRY(device_fault_check(s));
+    if (where == RTM_HOST || !stream) RTM_TRY(fault_check(s, {pc->op.get()}));
     return RTM_OK;
 }
 
@@ -756,7 +756,7 @@ int rtm_plate_batch_apply(rtm_plate_batch* b, int preconditioner, const void* x,
     RTM_TRY(op->apply(in.ptr, o.ptr, count, s, SkipFlags{}));
     RTM_TRY(out_finish(y, total, prec, where, o, s));
     if (where == RTM_HOST || !stream) RTM_CUDA(cudaStreamSynchronize(s));
-    return device_fault_check(s);
+    return fault_check(s, {op});
 }
 
 int rtm_plate_batch_solve(rtm_plate_batch* b, const rtm_solve_config* config, const void* rhs, const void* x0,

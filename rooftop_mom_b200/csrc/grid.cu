@@ -535,8 +535,8 @@ int apply_plate_batch(const std::vector<const GridApplicator*>& plates, const vo
 
 int GridApplicator::apply(const void* x, void* y, int nrhs, cudaStream_t s, SkipFlags skip) {
     if (nrhs < 1 || nrhs > max_rhs) return fail(RTM_ERR_ARG, "more right-hand sides than the product reserved");
-    return precision == RTM_FP64 ? apply_t<double>(*this, x, y, nrhs, s, skip, work.ptr, fault)
-                                 : apply_t<float>(*this, x, y, nrhs, s, skip, work.ptr, fault);
+    return precision == RTM_FP64 ? apply_t<double>(*this, x, y, nrhs, s, skip, work.ptr, fault.ptr)
+                                 : apply_t<float>(*this, x, y, nrhs, s, skip, work.ptr, fault.ptr);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -556,8 +556,8 @@ int apply_fixed_scratch(const GridApplicator& g, const void* x, void* y, int nrh
                                       std::to_string(cap) + " bytes");
     void* work = nullptr;
     if (g.mode != kStrip) RTM_TRY(fixed_scratch_address(&work));
-    return g.precision == RTM_FP64 ? apply_t<double>(g, x, y, nrhs, s, SkipFlags{}, work, g.fault)
-                                   : apply_t<float>(g, x, y, nrhs, s, SkipFlags{}, work, g.fault);
+    return g.precision == RTM_FP64 ? apply_t<double>(g, x, y, nrhs, s, SkipFlags{}, work, g.fault.ptr)
+                                   : apply_t<float>(g, x, y, nrhs, s, SkipFlags{}, work, g.fault.ptr);
 }
 
 // ============================================================================================
@@ -741,7 +741,7 @@ int build_product(const DeviceGenerators& g, double size_x, double size_y, int p
     out.max_rhs = std::max(1, max_rhs);
     out.lean = product == RTM_PRODUCT_LEAN;
     if (out.content == RTM_NONE) return fail(RTM_ERR_ARG, "a single face carries no rooftop");
-    RTM_TRY(device_fault_word(&out.fault));  // may allocate pinned memory: here, as a first apply may run under capture
+    RTM_TRY(out.fault.acquire());
     GenArgs a{};
     a.kind = kSrcEmbed;
     if (product == RTM_PRODUCT_FFT) {
@@ -1179,7 +1179,7 @@ int build_circulant(const DeviceGenerators& g, double size_x, double size_y, int
     out.size_x = size_x;
     out.size_y = size_y;
     out.max_rhs = 1;
-    RTM_TRY(device_fault_word(&out.fault));
+    RTM_TRY(out.fault.acquire());
     out.P = cx;
     out.Q = cy;
     out.nsx = out.nsy = 1;

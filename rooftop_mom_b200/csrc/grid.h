@@ -56,7 +56,7 @@ struct GridApplicator : LinearOp {
     DeviceBuffer spec;      // GEN3: [sub][3][Q][P]; BLOCK4: [4][Q][P]; STRIP: [sub][P]
     DeviceBuffer work;      // W
     int spec_blocks = 0;    // blocks stored
-    int* fault = nullptr;   // the device's fault word, looked up when the product is built: a first apply may run under capture
+    FaultWord fault;        // taken when the product is built: a first apply may run under capture
     FastSchedule sched;     // schedule of the power-of-two kernels (set when the product is built)
 
     // y = A x on the device for nrhs vectors of length n (precision of the product).
@@ -65,6 +65,7 @@ struct GridApplicator : LinearOp {
     size_t work_bytes_per_rhs() const;
     double stored_bytes() const override { return (double)spec.bytes; }
     double working_bytes() const override { return (double)work.bytes; }
+    bool take_fault() override { return fault.take(); }
 };
 
 // Plate batches (several plates, one right-hand side each, in one launch of each kernel): whether a

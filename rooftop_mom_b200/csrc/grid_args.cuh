@@ -49,7 +49,7 @@ template <typename T> struct GridArgs {
     const int* skip;  // per right-hand side, nonzero: leave it alone
     int skip_stride;
     int cb, ls;  // x-mix: y frequencies per CTA and the padded line stride
-    int* fault;  // the device's fault word: set to RTM_ERR_TIMEOUT by a bounded wait that ran out
+    int* fault;  // the operator's fault word: set to RTM_ERR_TIMEOUT by a bounded wait that ran out
     const PlateDesc<T>* plates;  // plate batch: per right-hand side (device); null: every one on this plate
 };
 

@@ -175,11 +175,17 @@ void extracted_moments(double size_x, double size_y, double k, double out[7][4])
 
 int fast_fft_size(int count);
 
-// The device's fault word, which kernels with bounded waits set to RTM_ERR_TIMEOUT when a wait runs out (pinned host
-// memory mapped by the devices; the first lookup of a process allocates it, so it is made outside any stream
-// capture), and its check: synchronises the stream, reads and clears the word, and returns RTM_ERR_TIMEOUT if it was
-// set.
-int device_fault_word(int** out);
-int device_fault_check(cudaStream_t s);
+// An operator's fault word, which its kernels with bounded waits set to RTM_ERR_TIMEOUT when a wait runs out: pinned
+// host memory mapped by the devices. acquire() may allocate, so it is called when the operator is built, outside any
+// stream capture; take() reads and clears the word, after a synchronisation.
+struct FaultWord {
+    int* ptr = nullptr;
+    FaultWord() = default;
+    FaultWord(const FaultWord&) = delete;
+    FaultWord& operator=(const FaultWord&) = delete;
+    ~FaultWord();
+    int acquire();
+    bool take();
+};
 
 }  // namespace rtm

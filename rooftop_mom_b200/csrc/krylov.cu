@@ -1847,7 +1847,7 @@ static int cocg(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* bv
     res.history.resize((size_t)hs * nrhs);
     RTM_CUDA(cudaMemcpyAsync(res.history.data(), hist.ptr, hist.bytes, cudaMemcpyDeviceToHost, s));
     RTM_CUDA(cudaStreamSynchronize(s));
-    RTM_TRY(device_fault_check(s));
+    RTM_TRY(fault_check(s, {A, M}));
     res.hist_stride = hs;
     res.stats.resize(nrhs);
     for (int k = 0; k < nrhs; ++k) {
@@ -2046,7 +2046,7 @@ static int gmres(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b
     res.history.resize((size_t)hs * nrhs);
     RTM_CUDA(cudaMemcpyAsync(res.history.data(), hist.ptr, hist.bytes, cudaMemcpyDeviceToHost, s));
     RTM_CUDA(cudaStreamSynchronize(s));
-    RTM_TRY(device_fault_check(s));
+    RTM_TRY(fault_check(s, {A, M}));
     res.hist_stride = hs;
     res.stats.resize(nrhs);
     for (int k = 0; k < nrhs; ++k) {
@@ -2247,7 +2247,7 @@ int solve_mixed(LinearOp* A64, LinearOp* A32, LinearOp* M32, const SolveConfig& 
         count_launch();
         RTM_CUDA(cudaStreamSynchronize(s));
     }
-    RTM_TRY(device_fault_check(s));
+    RTM_TRY(fault_check(s, {A64, A32, M32, M64}));
     res.hist_stride = hs;
     res.stats.resize(nrhs);
     for (int k = 0; k < nrhs; ++k) {

@@ -1,6 +1,7 @@
 // Linear operators on rooftop vectors, as the solvers see them.
 #pragma once
 
+#include <initializer_list>
 #include <memory>
 
 #include "internal.h"
@@ -23,7 +24,12 @@ struct LinearOp {
     virtual int reserve(int nrhs) { (void)nrhs; return RTM_OK; }
     virtual double stored_bytes() const { return 0; }
     virtual double working_bytes() const { return 0; }
+    // Whether a wait of the operator's kernels has run out since the last call (their stream synchronised before).
+    virtual bool take_fault() { return false; }
 };
+
+// Synchronises the stream and takes the operators' faults (null entries aside): RTM_ERR_TIMEOUT if there was one.
+int fault_check(cudaStream_t s, std::initializer_list<LinearOp*> ops);
 
 // Dense n x n complex FP64 matrix (column-major).
 std::unique_ptr<LinearOp> make_dense_op(const double2* device_matrix, int64_t n, int* status);

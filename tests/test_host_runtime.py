@@ -1,0 +1,40 @@
+"""The library's host runtime (runtime.cpp, fault.cu) compiled against a stand-in for the CUDA runtime
+(tests/c/host_runtime.cpp), so that what it allocates, copies and reports is checked without a GPU."""
+from __future__ import annotations
+
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    from rooftop_mom_b200 import build
+
+    if shutil.which("g++") is None:
+        pytest.skip("no C++ compiler")
+    exe = str(tmp_path_factory.mktemp("c") / "host_runtime")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(build._nvcc())), "include")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-I", cuda, "-x", "c++", os.path.join(ROOT, "tests", "c", "host_runtime.cpp"),
+                    os.path.join(build.CSRC, "runtime.cpp"), os.path.join(build.CSRC, "fault.cu"), "-o", exe], check=True,
+                   capture_output=True, text=True)
+
+    def go(*args):
+        out = subprocess.run([exe, *args], check=True, capture_output=True, text=True, timeout=120).stdout
+        return {line.split()[0]: line.split()[1:] for line in out.splitlines()}
+
+    return go
+
+
+def test_a_fault_is_reported_by_its_own_operator(run):
+    from rooftop_mom_b200 import _lib as L
+
+    got = run("faults")
+    assert got["other"] == ["0"]
+    assert got["own"] == [str(L.ERR_TIMEOUT)]
+    assert got["again"] == ["0"]
+    assert got["reused"] == ["0", "pages", "1"]
