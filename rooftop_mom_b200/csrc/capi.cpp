@@ -173,7 +173,7 @@ int rtm_launch_count(int64_t* count) {
     return RTM_OK;
 }
 
-int rtm_budget_require(double bytes) { return budget_require(bytes, "The request"); }
+int rtm_budget_require(double bytes) { return budget_require(bytes, "The request", true); }
 
 int rtm_estimate_bytes(int count_x, int count_y, int product, int method, int preconditioned, int restart,
                        int max_iterations, double out[6]) {

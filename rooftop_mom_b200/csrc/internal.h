@@ -53,7 +53,8 @@ struct DeviceOnce {
 
 // ---------------------------------------------------------------------------------------------
 // Budget ledger of device bytes (Budget.m). Thread-safe.
-int budget_require(double bytes, const char* what);
+// fresh: no allocation of the bytes follows, so the device's free memory is read anew however small they are.
+int budget_require(double bytes, const char* what, bool fresh = false);
 // A byte count as the reference's messages write it (formatBytes.m): "512 B", "1.5 kB", "3.0 GB".
 std::string format_bytes(double bytes);
 void budget_hold(double bytes);

@@ -54,10 +54,12 @@ std::string format_bytes(double b) {
     return buf;
 }
 
-// The device's free memory as far as a request of `bytes` depends on it. cudaMemGetInfo takes 0.2 to 1 ms here (it
-// waits on the driver for all users of the machine) and every set-up and solve asks, so a reading decides requests of
-// up to a sixteenth of it for kReadingAge; larger requests and older readings read again. The library's own
-// allocations are taken off the reading. Called with g_budget_mu held.
+// The device's free memory as far as a request of `bytes` depends on it, for a request whose memory is allocated right
+// after the check: the allocation itself then refuses what other users of the device have taken since the reading, with
+// the same status. cudaMemGetInfo takes 0.2 to 1 ms in a process that uses torch and every set-up and solve asks, so a
+// reading decides such requests of up to a sixteenth of it for kReadingAge; larger requests and older readings read
+// again, and so does a check that nothing follows (fresh). The library's own allocations are taken off the reading. Called
+// with g_budget_mu held.
 constexpr double kReadingAge = 0.1;  // seconds
 struct FreeReading {
     double bytes = -1;
@@ -65,12 +67,12 @@ struct FreeReading {
 };
 static FreeReading g_free[64];
 
-static bool free_memory(double bytes, double* out) {
+static bool free_memory(double bytes, bool fresh, double* out) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     FreeReading& r = g_free[dev & 63];
     const auto now = std::chrono::steady_clock::now();
-    if (dev < 64 && r.bytes >= 16 * bytes && std::chrono::duration<double>(now - r.at).count() < kReadingAge) {
+    if (!fresh && dev < 64 && r.bytes >= 16 * bytes && std::chrono::duration<double>(now - r.at).count() < kReadingAge) {
         *out = r.bytes;
         return true;
     }
@@ -82,7 +84,7 @@ static bool free_memory(double bytes, double* out) {
     return true;
 }
 
-int budget_require(double bytes, const char* what) {
+int budget_require(double bytes, const char* what, bool fresh) {
     std::lock_guard<std::mutex> lk(g_budget_mu);
     if (g_ceiling > 0 && g_held + bytes > g_ceiling) {
         return fail(RTM_ERR_OOM_BUDGET, std::string(what) + " needs " + format_bytes(bytes) + ", but only " +
@@ -90,7 +92,7 @@ int budget_require(double bytes, const char* what) {
                                             " of the memory ceiling of " + format_bytes(g_ceiling) + " are left.");
     }
     double free_b = 0;
-    if (free_memory(bytes, &free_b) && bytes > free_b) {
+    if (free_memory(bytes, fresh, &free_b) && bytes > free_b) {
         return fail(RTM_ERR_OOM_BUDGET, std::string(what) + " needs " + format_bytes(bytes) + ", but only " +
                                             format_bytes(free_b) + " are free on this device.");
     }

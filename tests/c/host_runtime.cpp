@@ -63,8 +63,20 @@ static void faults() {
     std::printf("reused %d pages %d\n", fault_check(nullptr, {&d}), g_host_allocs);
 }
 
+// Memory that another user of the device takes between two checks.
+static void budget() {
+    const double gib = double(1 << 30);
+    std::printf("first %d\n", budget_require(gib, "The request", true));
+    g_free_bytes = size_t(1) << 29;
+    std::printf("taken %d\n", budget_require(gib, "The request", true));
+    DeviceBuffer b;
+    const int checked = budget_require(gib, "The product");
+    std::printf("allocated %d\n", checked != RTM_OK ? checked : b.alloc(size_t(1) << 30));
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "faults") faults();
+    if (what == "budget") budget();
     return 0;
 }

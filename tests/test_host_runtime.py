@@ -38,3 +38,14 @@ def test_a_fault_is_reported_by_its_own_operator(run):
     assert got["own"] == [str(L.ERR_TIMEOUT)]
     assert got["again"] == ["0"]
     assert got["reused"] == ["0", "pages", "1"]
+
+
+def test_memory_that_others_take_is_refused_at_once(run):
+    """A request that fitted is refused when another user of the device has taken the memory meanwhile: by the check
+    itself where nothing is allocated after it (rtm_budget_require), else at the latest by the allocation."""
+    from rooftop_mom_b200 import _lib as L
+
+    got = run("budget")
+    assert got["first"] == ["0"]
+    assert got["taken"] == [str(L.ERR_OOM_BUDGET)]
+    assert got["allocated"] == [str(L.ERR_OOM_BUDGET)]
