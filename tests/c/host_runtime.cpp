@@ -1,9 +1,12 @@
 // The host side of the library (runtime.cpp, fault.cu) on a stand-in for the CUDA runtime that only counts and copies, so
 // that it runs without a GPU. Prints "<name> <values>" a line; the first argument names the scenario.
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <vector>
 
 #include "../../rooftop_mom_b200/csrc/ops.h"
 
@@ -74,9 +77,78 @@ static void budget() {
     std::printf("allocated %d\n", checked != RTM_OK ? checked : b.alloc(size_t(1) << 30));
 }
 
+// The tables of a length against their definitions in long double: the largest error of each precision, relative to the
+// largest entry of its table, and the allocations and copies that they took.
+static double g_err64 = 0, g_err32 = 0;
+template <typename F> static void compare(const double2* a, const float2* b, int count, F&& want) {
+    long double most = 0, e64 = 0, e32 = 0;
+    for (int i = 0; i < count; ++i) {
+        long double re, im;
+        want(i, re, im);
+        most = std::max(most, hypotl(re, im));
+        e64 = std::max(e64, hypotl(a[i].x - re, a[i].y - im));
+        e32 = std::max(e32, hypotl(b[i].x - re, b[i].y - im));
+    }
+    g_err64 = std::max(g_err64, (double)(e64 / most));
+    g_err32 = std::max(g_err32, (double)(e32 / most));
+}
+
+static const long double kPi = 3.141592653589793238462643383279502884L;
+
+// exp(-i pi num / den)
+static void root(long double num, long double den, long double& re, long double& im) {
+    re = cosl(kPi * num / den);
+    im = -sinl(kPi * num / den);
+}
+
+static void bluestein(int n, int m, const double2* chirp64, const float2* chirp32, const double2* kern64,
+                      const float2* kern32, const double2* tw64, const float2* tw32) {
+    compare(chirp64, chirp32, n, [&](int j, long double& re, long double& im) { root((long long)j * j % (2 * n), n, re, im); });
+    compare(tw64, tw32, m, [&](int k, long double& re, long double& im) { root(2 * k, m, re, im); });
+    std::vector<long double> c(2 * n), w(2 * m);
+    for (int j = 0; j < n; ++j) root((long long)j * j % (2 * n), n, c[2 * j], c[2 * j + 1]);
+    for (int k = 0; k < m; ++k) root(2 * k, m, w[2 * k], w[2 * k + 1]);
+    compare(kern64, kern32, m, [&](int k, long double& re, long double& im) {
+        re = im = 0;
+        for (int j = -(n - 1); j < n; ++j) {
+            const int d = std::abs(j), e = (int)(((long long)(j + m) * k) % m);  // conj(c_|j|) w^(j k)
+            re += c[2 * d] * w[2 * e] + c[2 * d + 1] * w[2 * e + 1];
+            im += c[2 * d] * w[2 * e + 1] - c[2 * d + 1] * w[2 * e];
+        }
+        re /= m;
+        im /= m;
+    });
+}
+
+static void tables(int n) {
+    const FftTables* t = nullptr;
+    g_mallocs = g_copies = 0;
+    const int st = fft_tables(n, &t);
+    std::printf("cost %d %d %d\n", st, g_mallocs, g_copies);
+    if (st != RTM_OK) return;
+    compare(t->tw64, t->tw32, n, [&](int k, long double& re, long double& im) { root(2 * k, n, re, im); });
+    compare(t->mod64, t->mod32, n, [&](int k, long double& re, long double& im) { root(k, n, re, im); });
+    const FftPlan& p = t->plan;
+    const RegPlan& r = t->reg;
+    if (p.m != n) bluestein(n, p.m, p.chirp64, p.chirp32, p.kern64, p.kern32, p.twm64, p.twm32);
+    if (r.n1 && r.m != n) bluestein(n, r.m, r.chirp64, r.chirp32, r.kern64, r.kern32, r.tw64, r.tw32);
+    if (r.n1 && r.m == n) compare(r.tw64, r.tw32, n, [&](int k, long double& re, long double& im) { root(2 * k, n, re, im); });
+    if (t->ta64) {
+        compare(t->ta64, t->ta32, n, [&](int i, long double& re, long double& im) { root(2 * (i / r.n2) * (i % r.n2), n, re, im); });
+        compare(t->tb64, t->tb32, n, [&](int i, long double& re, long double& im) { root(2 * (i / r.n1) * (i % r.n1), n, re, im); });
+    }
+    if (t->t364) {
+        compare(t->t364, t->t332, n, [&](int i, long double& re, long double& im) { root(2 * (i / 64) * (i % 64), n, re, im); });
+        compare(t->t364 + n, t->t332 + n, 64, [&](int i, long double& re, long double& im) { root(2 * (i / 8) * (i % 8), 64, re, im); });
+    }
+    std::printf("kind %d %d %d\n", p.m != n, r.n1 ? r.m != n : -1, (t->ta64 != nullptr) + (t->t364 != nullptr));
+    std::printf("errors %.3e %.3e\n", g_err64, g_err32);
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "faults") faults();
     if (what == "budget") budget();
+    if (what == "tables") tables(std::atoi(argv[2]));
     return 0;
 }

@@ -49,3 +49,21 @@ def test_memory_that_others_take_is_refused_at_once(run):
     assert got["first"] == ["0"]
     assert got["taken"] == [str(L.ERR_OOM_BUDGET)]
     assert got["allocated"] == [str(L.ERR_OOM_BUDGET)]
+
+
+@pytest.mark.parametrize(
+    "n,kind",  # Bluestein in the Stockham engine; on register-resident lines (-1: none); sets of reordered twiddles
+    [(1, (0, -1, 0)), (12, (0, 0, 0)), (13, (0, -1, 0)), (22, (0, 1, 0)), (32, (0, 0, 1)), (67, (1, 1, 0)), (97, (1, 1, 0)),
+     (128, (0, 0, 1)), (256, (0, 0, 2)), (499, (1, 1, 0)), (509, (1, 1, 0)), (521, (1, -1, 0)), (1000, (0, -1, 0)),
+     (1024, (0, 0, 2))],
+)
+def test_the_tables_of_a_length_take_one_allocation_and_one_copy(run, n, kind):
+    """A set-up at a length new to the process pays for its tables: one device allocation, one copy, and entries within
+    their rounding (half a unit in the last place of each part, 2^-53 sqrt(2) and 2^-24 sqrt(2), relative to the table's
+    largest entry; FP32 entries are rounded twice)."""
+    got = run("tables", str(n))
+    assert got["cost"] == ["0", "1", "1"]
+    assert tuple(int(v) for v in got["kind"]) == kind
+    e64, e32 = (float(v) for v in got["errors"])
+    assert e64 <= 1.01 * 2**-53 * 2**0.5
+    assert e32 <= 1.01 * 2**-24 * 2**0.5
