@@ -15,7 +15,9 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "librtm.so")
 OBJ = os.path.join(HERE, "_build")
 SOURCES = ["runtime.cpp", "capi.cpp", "server.cpp", "grid.cu", "grid_fast.cu", "assembly.cu", "krylov.cu", "strip_solve.cu", "ops.cu", "excitation.cu", "fixed_scratch.cu", "fault.cu", "tune.cpp", "batch.cu"]
-# sources compiled once for each form, so that their kernels compile side by side: object name -> (source, defines)
+# Sources compiled once for each form, so that their kernels compile side by side: object name -> (source, defines).
+# Without -lineinfo: a kernel's first launch in a process loads its whole unit, and the line tables of the unrolled
+# codelets are three quarters of these (first product on 250 x 139 faces 27 ms with them, 7 without; librtm.so 84 MB, 41).
 FORMS = {**{f"grid_reg.{k}": ("grid_reg.cu", [f"-DRTM_REG_FORM={k}"]) for k in range(8)},
          **{f"gen_reg.{k}": ("gen_reg.cu", [f"-DRTM_GEN_FORM={k}"]) for k in range(4)}}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -48,7 +50,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         path = os.path.join(CSRC, src)
         obj = os.path.join(OBJ, name + ".o")
         if force or _stale(obj, [path] + headers):
-            cmd = [nvcc, *FLAGS, *ARCH, *defines, "-c", path, "-o", obj]
+            flags = [f for f in FLAGS if f != "-lineinfo" or name not in FORMS]
+            cmd = [nvcc, *flags, *ARCH, *defines, "-c", path, "-o", obj]
             jobs.append((name, cmd))
 
     def run(job):
