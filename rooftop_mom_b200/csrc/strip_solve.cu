@@ -19,7 +19,7 @@ namespace rtm {
 namespace {
 
 constexpr int kStripThreads = 256;
-constexpr int kStripLaunch = 512;  // iterations a launch runs at most (the host checks for a cancel between launches)
+constexpr int kStripLaunch = 512;  // iterations a launch runs at most, where no cancel can arrive
 constexpr size_t kStripSmem = 200 * 1024;
 
 // One strip product: ns subbands of a line of plan.n points (k_strip in grid.cu).
@@ -275,7 +275,6 @@ int strip_cocg(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b, 
     a.has_x0 = x0 != nullptr;
     a.tol = cfg.tolerance;
     a.max_iterations = cfg.max_iterations;
-    a.limit = kStripLaunch;
     static DeviceOnce once;
     RTM_TRY(once([]() -> int {
         RTM_CUDA(cudaFuncSetAttribute(k_strip_cocg<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStripSmem));
@@ -305,16 +304,24 @@ int strip_cocg(LinearOp* A, LinearOp* M, const SolveConfig& cfg, const void* b, 
     a.st = reinterpret_cast<StripState*>(back.as<char>() + hist_bytes);
     std::vector<char> host(back_bytes);
     const auto* st = reinterpret_cast<const StripState*>(host.data() + hist_bytes);
-    for (int launched = 0;; launched += kStripLaunch) {
-        a.first = launched == 0;
+    // a cancel is looked for before the first iteration and after every check_every (krylov.cu's cocg does the same)
+    const int limit = !cfg.cancel ? kStripLaunch : cfg.check_every > 0 ? cfg.check_every : 16;
+    const bool small = hist_bytes <= 16 * 1024;  // the history comes back with every look at the states, or once
+    for (a.first = 1;; a.first = 0) {
+        a.limit = cfg.cancel && *cfg.cancel ? 0 : limit;
         k_strip_cocg<T><<<nrhs, kStripThreads, smem, s>>>(a);
         count_launch();
         RTM_CUDA(cudaGetLastError());
-        RTM_CUDA(cudaMemcpyAsync(host.data(), back.ptr, back_bytes, cudaMemcpyDeviceToHost, s));
+        const size_t from = small ? 0 : hist_bytes;
+        RTM_CUDA(cudaMemcpyAsync(host.data() + from, back.as<char>() + from, back_bytes - from, cudaMemcpyDeviceToHost, s));
         RTM_CUDA(cudaStreamSynchronize(s));
         bool all = true;
         for (int k = 0; k < nrhs; ++k) all = all && st[k].done;
         if (all || (cfg.cancel && *cfg.cancel)) break;
+    }
+    if (!small) {
+        RTM_CUDA(cudaMemcpyAsync(host.data(), back.ptr, hist_bytes, cudaMemcpyDeviceToHost, s));
+        RTM_CUDA(cudaStreamSynchronize(s));
     }
     const auto* hist = reinterpret_cast<const double*>(host.data());
     res.history.assign(hist, hist + (size_t)hs * nrhs);
