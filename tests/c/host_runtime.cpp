@@ -145,10 +145,19 @@ static void tables(int n) {
     std::printf("errors %.3e %.3e\n", g_err64, g_err32);
 }
 
+// The split of every length that has one: "<n> <n1> <n2> <m>", m == n without a Bluestein convolution.
+static void splits() {
+    for (int n = 2; n <= kRegMax; ++n) {
+        const FftTables* t = nullptr;
+        if (fft_tables(n, &t) == RTM_OK && t->reg.n1) std::printf("%d %d %d %d\n", n, t->reg.n1, t->reg.n2, t->reg.m);
+    }
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "faults") faults();
     if (what == "budget") budget();
+    if (what == "splits") splits();
     if (what == "tables") tables(std::atoi(argv[2]));
     return 0;
 }

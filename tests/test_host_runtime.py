@@ -67,3 +67,20 @@ def test_the_tables_of_a_length_take_one_allocation_and_one_copy(run, n, kind):
     e64, e32 = (float(v) for v in got["errors"])
     assert e64 <= 1.01 * 2**-53 * 2**0.5
     assert e32 <= 1.01 * 2**-24 * 2**0.5
+
+
+def test_the_codelet_lengths_reach_every_case_of_the_splits(run):
+    """test_gpu_codelets.LENGTHS take every first and second factor that any length up to 1024 has, by register class
+    (first factors up to 16, or above), with and without a Bluestein convolution: each is a case of its own in the
+    kernels' switches."""
+    from test_gpu_codelets import LENGTHS
+
+    def cases(n):
+        n1, n2, m = (int(v) for v in splits[str(n)])
+        return {(m != n, n1 > 16, "first", n1), (m != n, n1 > 16, "second", n2)}
+
+    splits = run("splits")
+    assert len(splits) > 500
+    every = set().union(*(cases(int(n)) for n in splits))
+    assert set().union(*(cases(n) for n in LENGTHS)) == every
+    assert min(int(n) for n in splits) in LENGTHS and max(int(n) for n in splits) in LENGTHS
