@@ -409,8 +409,9 @@ def plane_wave_vectors(theta_deg, phi_deg, pol):
 
 
 def matvec_bytes(n_unknowns, P, Q, elem):
-    """Algorithmic bytes of one split-FFT product (2-pass schedule): e (2N + 16 PQ + 12 PQ)."""
-    return elem * (2 * n_unknowns + 16 * P * Q + 12 * P * Q)
+    """Algorithmic bytes of one split-FFT product (2-pass schedule): e (2N + 16 PQ + 3 (P + 1)(Q + 1)). The spectra are
+    even in both frequencies, so of their 12 PQ stored values 3 (P + 1)(Q + 1) are distinct, and a product reads those."""
+    return elem * (2 * n_unknowns + 16 * P * Q + 3 * (P + 1) * (Q + 1))
 
 
 class Clocks:
@@ -829,8 +830,8 @@ def run_reference_full(args, w):
 METRIC = "solves/s at rel. residual 1e-6, mixed vs FP64 GPU; matvec HBM GB/s; p99 ms"
 
 # DRAM bytes (read + write) of one product, summed over its three kernels, from one ncu capture each
-# (profiles/product_fast_path.md); None where no capture was made.
-TRAFFIC = {"c2": 23.2e6, "c3": 200.3e6}
+# (profiles/product_three_steps.md); None where no capture was made.
+TRAFFIC = {"c2": 13.8e6, "c3": 112.3e6}
 
 
 def config_of(args, w):
