@@ -166,17 +166,19 @@ typedef struct rtm_tune_result {
     int fft_x, fft_y;          /* chosen transform grid */
     int y_blocks, mix_kind;    /* chosen schedule: CTAs per SM of the y passes (1..3) and the x-mix form
                                   (0..2 direct with 1..3 CTAs per SM, 3 pipelined); 0 and -1 off the
-                                  power-of-two path */
+                                  power-of-two path. Along an axis of length 256 or 512 (FP64), 512 or 1024
+                                  (FP32), y_blocks 1 and mix_kind 0 stand for the three-step form of the
+                                  transforms, with CTAs per SM of its own, in place of one CTA per SM */
     double seconds;            /* device time of one product (nrhs vectors) with the choice */
     double reference_seconds;  /* the same with the reference's sizes and the default schedule */
     int candidates;            /* configurations measured */
 } rtm_tune_result;
 RTM_API int rtm_tune_product(int count_x, int count_y, int precision, int nrhs, int flags, rtm_tune_result* out);
-/* Forgets every choice of the autotuner (products created afterwards take the reference's sizes). */
 /* Records fft_x x fft_y (at least the face counts) as the transform grid of the split products built
  * afterwards for this face grid and precision on the calling thread's device, with the default kernel
  * schedule, as if the autotuner had chosen it (e.g. powers of two for plates that go into one batch). */
 RTM_API int rtm_tune_set(int count_x, int count_y, int precision, int fft_x, int fft_y);
+/* Forgets every choice of the autotuner (products created afterwards take the reference's sizes). */
 RTM_API int rtm_tune_clear(void);
 
 /* A dense n x n complex operator (column-major), for solving any small system with the same solvers

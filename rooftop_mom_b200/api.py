@@ -784,7 +784,8 @@ def tuneProduct(mesh: Mesh, precision="double", nrhs: int = 1, flushL2: bool = T
     """Autotunes the split product of a plate (rtm_tune_product): measures the candidate transform grids (the
     reference's 7-smooth sizes, generateFastFFTSize.m, and the next powers of two) and kernel schedules on the
     device and keeps the fastest for the operators created afterwards for this face grid and precision.
-    Returns the choice and its time beside the reference sizes' time."""
+    Returns the choice and its time beside the reference sizes' time; yBlocks and mixKind as in rtm_tune_result
+    (1 and 0 stand for the three-step transforms along an axis of a length that has them)."""
     if precision not in L.PRECISIONS:
         raise _err("rooftopMoM:operator:invalidPrecision", "The precision is 'double' or 'single'.")
     cx, cy = mesh.count()

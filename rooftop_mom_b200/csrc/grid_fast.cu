@@ -334,10 +334,11 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_y_fwd(const Gri
 // 25 MB instead of 100).
 __device__ __forceinline__ int even_freq(int m, int p, int n) { return min(m, n - m - p); }
 
-// The R2 <= 32 threads of an x line are lanes of one warp, so its exchanges need no CTA barrier. FP32 takes that (1024 x
-// 1024 product 128 -> 125 us, eight 512 x 512 ones 199 -> 190); FP64, whose CTAs hold four warps with up to 255
-// registers, keeps the barriers: its warps then share the twiddle and spectra lines (512 x 512 product 51 us without
-// them, 47 with).
+// The R2 <= 32 threads of an x line are lanes of one warp, so its exchanges need no CTA barrier. FP32 takes that, and
+// shuffles for the partner's values (products of 256 x 256: 12.1 us, 12.6 with barriers, four vectors 23.2 against
+// 24.7; 64 x 64 7.4 against 7.9; 128 x 128 alone 13.2 against 12.9). FP64, whose CTAs hold four warps with up to 255
+// registers, keeps the barriers: its warps then share the twiddle and spectra lines (512 x 512 in two steps: 47 us, 51
+// without them).
 template <typename T> __device__ __forceinline__ void line_sync() {
     if constexpr (sizeof(T) == 8) __syncthreads();
     else __syncwarp();
@@ -446,15 +447,13 @@ __global__ void __launch_bounds__(Fast<T>::threads, MINB) k_fast_x_mix_direct(co
     }
 }
 
-// The lengths of split products that run in three steps, a thread holding both components of an x line (they share the
-// twiddles, the phases and E, and meet in registers) or both subbands of a column; the small radices need half the
-// registers. The L1 pipe bounds both forms of the x-mix (FP64 512 x 512 with four vectors: 49 % busy at 8 warps an SM
-// before, 70 % now). Product, two steps -> three, one vector and four: FP64 256 x 256 15.9 -> 13.5 us and 42.9 -> 36.8; 512
-// x 512 46.6 -> 37.2 and 185 -> 139; FP32 512 x 512 29.6 -> 25.2 and 94 -> 81; 1024 x 1024 104 -> 89 and 382 -> 345. FP32
-// 256 x 256 stays on two steps (x-mix in three: 12.5 against 12.4 us, 24.9 against 23.4): its lines exchange within their
-// warps there; shorter lines leave too few threads for three steps. Without subbands every such length gains, FP32 256 too
-// (circulants, against the register-resident lines of grid_reg.cu: FP64 256 x 256 20.5 -> 11.3, 512 x 512 35.2 -> 17.3;
-// FP32 17.9 -> 10.1, 27.9 -> 15.4, 1024 x 1024 110 -> 36).
+// The lengths that run in three steps by default when both lengths of a split product are powers of two, a thread
+// holding both components of an x line (they share the twiddles, the phases and E, and meet in registers) or both subbands
+// of a column; the small radices need half the registers. The L1 pipe bounds both forms of the x-mix (FP64 512 x 512 with
+// four vectors: 49 % busy in two steps at 8 warps an SM, 70 % in three). Product, two steps -> three, one vector and four:
+// FP64 256 x 256 15.9 -> 13.5 us and 42.9 -> 36.8; 512 x 512 46.6 -> 37.2 and 185 -> 139; FP32 512 x 512 29.6 -> 25.2 and
+// 94 -> 81; 1024 x 1024 104 -> 89 and 382 -> 345. FP32 256 x 256 stays on two steps (x-mix in three: 12.5 against 12.4 us,
+// 24.9 against 23.4): its lines exchange within their warps there; shorter lines leave too few threads for three steps.
 constexpr bool three_step(int n, bool fp64) { return fp64 ? n == 256 || n == 512 : n == 512 || n == 1024; }
 
 // SUB: the subbands along x (2: a split product, 1: an embedding or a circulant).
@@ -1080,6 +1079,11 @@ template <typename T> int dispatch_x(const GridArgs<T>& a, int nrhs, int kind, c
 
 }  // namespace
 
+// The lengths whose passes run in three steps where the other choice is the register-resident lines of grid_reg.cu, with
+// no two-step form beside them: FP32 256 gains there too. Circulants, lines of grid_reg.cu -> three steps: FP64 256 x 256
+// 20.5 -> 11.3 us, 512 x 512 35.2 -> 17.3; FP32 17.9 -> 10.1, 27.9 -> 15.4, 1024 x 1024 110 -> 36. FP32 split products with
+// one length of 256, one vector and four: 256 x 35 17.6 -> 8.4 and 19.6 -> 12.7, 256 x 700 33.0 -> 29.5 and 80.7 ->
+// 68.2, 100 x 256 16.9 -> 12.4 and 19.9 -> 18.0.
 bool three_step_length(int n, bool fp64) { return n == 256 || n == 512 || (!fp64 && n == 1024); }
 
 namespace {

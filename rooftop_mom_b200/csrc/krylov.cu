@@ -96,8 +96,9 @@ __device__ __forceinline__ double2 cta_total(const double2* p, int nb) {
 }
 
 // The rows of a CTA in COCG's kernels: kRowChunk consecutive ones where the launch has a CTA for every chunk (up to
-// 592 of them), a grid stride above. The chunks' sums then add in one order whatever n, so a plate in a batch (whose
-// vectors end in zeros up to the batch's stride) takes the same iterations to the last bit as alone.
+// 592 of them, 303104 rows), a grid stride above. The chunks' sums then add in one order whatever n, so a plate in a
+// batch, whose vectors end in zeros up to the batch's stride, sums as it does alone (strips aside, which strip_solve.cu
+// solves alone and these kernels in a batch).
 constexpr int kRowChunk = 2 * kRT;
 struct Rows {
     int64_t first, end, step;

@@ -1,7 +1,7 @@
 // Register-resident transforms of lines of n = n1 n2 points (device code only), n1 >= n2 both codelet lengths of
-// at most 36. Every 7-smooth length from 16 to 1024 but 343, 686, 882 and 1000 has such a split; a length that has
-// none and is at most 512 runs as a Bluestein convolution on a length m = n1 n2 >= 2 n - 1, the others take the
-// Stockham engine of fft.cuh (make_reg_plan, runtime.cpp).
+// at most 36. 12, 15 and every 7-smooth length from 16 to 1024 but 343, 686, 882 and 1000 have such a split; a length with
+// a larger prime factor from 17 to 512 runs as a Bluestein convolution on a length m = n1 n2 >= 2 n - 1, the others take
+// the Stockham engine of fft.cuh (make_reg_plan, runtime.cpp).
 //
 // The four-step form: thread t < n2 of a line holds x[n2 m1 + t] (the "A" layout),
 //   reg_a_fwd: n1-point DFT over m1 in registers, twiddle w^(t k1), written to buf(k1, t);
