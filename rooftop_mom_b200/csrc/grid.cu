@@ -432,7 +432,7 @@ static int apply_t(const GridApplicator& g, const void* xv, void* yv, int nrhs, 
     int cb = 8;
     while (cb > 1 && (x_smem(cb) > (size_t)kSmemBudget || fft_threads(cb * g.nsx * 2, g.tP->plan) > kMaxThreads))
         cb /= 2;
-    while (cb > 1 && (int64_t)((g.Q + cb - 1) / cb) * npy * nrhs < 148) cb /= 2;
+    while (cb > 1 && (int64_t)((g.Q + cb - 1) / cb) * npy * nrhs < kDeviceSms) cb /= 2;
     const int ls = line_stride(g.tP->plan.m, cb * g.nsx * 2, elem);
     const int thr_x = fft_threads(cb * g.nsx * 2, g.tP->plan);
     if (y_smem(ti) > (size_t)kSmemBudget || x_smem(cb) > (size_t)kSmemBudget || thr_y > kMaxThreads ||

@@ -1033,7 +1033,7 @@ template <typename T, int NP> int launch_x_pipe(const GridArgs<T>& a, int nrhs, 
         return RTM_OK;
     }));
     const int iters = nrhs * 2 * (a.Q / M::TEAMS);
-    const int resident = dev >= 0 && dev < 64 && per_sm[dev] > 0 ? per_sm[dev] : 148;
+    const int resident = dev >= 0 && dev < 64 && per_sm[dev] > 0 ? per_sm[dev] : kDeviceSms;
     const int grid = std::max(1, std::min(iters, resident));
     RTM_CUDA(launch_dependent(k_fast_x_mix_pipe<T, NP>, dim3(grid), dim3(Fast<T>::threads), M::smem, s, a, iters));
     count_launch();

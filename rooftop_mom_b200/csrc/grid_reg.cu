@@ -403,7 +403,7 @@ int launch_reg_pass(int pass, GridArgs<T> a, const RegPlan& r, int nrhs, const v
         const int per = 2 * a.nsx * r.n1;
         a.ls = r.n1 * (r.n2 | 1);
         int cb = std::max(1, std::min(a.Q, kThreads / per));
-        while (cb > 1 && (int64_t)((a.Q + cb - 1) / cb) * a.npy * nrhs < 2 * 148) --cb;
+        while (cb > 1 && (int64_t)((a.Q + cb - 1) / cb) * a.npy * nrhs < 2 * kDeviceSms) --cb;
         a.cb = cb;
         const int threads = (cb * per + 31) / 32 * 32;
         const size_t smem = (size_t)cb * 2 * a.nsx * a.ls * sizeof(C2);

@@ -31,6 +31,10 @@ inline int check_cuda(cudaError_t e, const char* what) { return e == cudaSuccess
         if (s_ != RTM_OK) return s_;    \
     } while (0)
 
+// Streaming multiprocessors of a B200: what launch shapes are sized by. Kernels whose CTAs wait for one another ask the
+// device instead.
+constexpr int kDeviceSms = 148;
+
 extern int64_t g_launches;  // launches of this library's kernels (incremented by the launchers)
 inline void count_launch(int n = 1) { __atomic_fetch_add(&g_launches, (int64_t)n, __ATOMIC_RELAXED); }
 

@@ -867,7 +867,7 @@ __global__ void __launch_bounds__(kRT, 2) k_gm_orth_stream(const T2* __restrict_
 // CTAs and rows per CTA of k_gm_orth_stream: at least two CTAs per SM, chunks of at most about
 // kStreamRows rows, no more CTAs than the partial buffers hold.
 static void stream_config(int64_t n, int* blocks, int* chunk) {
-    const int64_t want = std::max<int64_t>(2 * 148, (n + kStreamRows - 1) / kStreamRows);
+    const int64_t want = std::max<int64_t>(2 * kDeviceSms, (n + kStreamRows - 1) / kStreamRows);
     const int64_t b = std::max<int64_t>(1, std::min<int64_t>(want, reduce_blocks(n)));
     int64_t c = (n + b - 1) / b;
     c = (c + 31) / 32 * 32;
@@ -921,7 +921,7 @@ template <typename T2> static void launch_orth(const T2* V, T2* w, int64_t n, in
     size_t smem;
     orth_config<T2>(ar.m, &TR, &smem);
     const int64_t tiles = (n + TR - 1) / TR;
-    const int blocks = (int)std::min<int64_t>({tiles, (int64_t)reduce_blocks(n), 2 * 148});
+    const int blocks = (int)std::min<int64_t>({tiles, (int64_t)reduce_blocks(n), 2 * kDeviceSms});
     k_gm_orth<T2><<<dim3(blocks, nrhs), kRT, smem, s>>>(V, w, n, nrhs, st, ar, mode, TR);
     count_launch();
 }
@@ -1418,7 +1418,7 @@ struct CgCluster {
     int ctas = 0, per = 0;
     CgCluster(int64_t n, int nrhs) {
         const int chunks = reduce_blocks(n);
-        if (n > kClusterRows || (chunks > 2 * kClusterMax && nrhs * kClusterMax > 148)) return;
+        if (n > kClusterRows || (chunks > 2 * kClusterMax && nrhs * kClusterMax > kDeviceSms)) return;
         ctas = 1;
         while (ctas < chunks && ctas < kClusterMax) ctas *= 2;
         per = 1;
@@ -1666,7 +1666,7 @@ void convert_to_fp64(const float2* in, double2* out, int64_t n, cudaStream_t s) 
     count_launch();
 }
 
-// CTAs of the vector kernels: about two elements per thread, at most 4 waves of the 148 SMs.
+// CTAs of the vector kernels: about two elements per thread, at most 4 waves of the SMs.
 static int reduce_blocks(int64_t n) {
     const int64_t b = (n + (int64_t)kRT * 2 - 1) / ((int64_t)kRT * 2);
     return (int)std::max<int64_t>(1, std::min<int64_t>(b, 592));
