@@ -383,13 +383,27 @@ __global__ void __launch_bounds__(kRT) k_gm_v0(const T2* __restrict__ w, T2* __r
     }
 }
 
-// The end of an Arnoldi step: the Hessenberg column col (its previous rotations applied) with the subdiagonal
-// ||w|| = sqrt(s), the new rotation, the rotated right-hand side, the history and the stopping tests (one thread).
-__device__ void arnoldi_rotate(GmState& S, GmArrays& ar, int rhs, double s, double2* col, double2* cs, double2* sn) {
+// The rest of an Arnoldi step once ||w|| is known: the Hessenberg column, its previous rotations,
+// the new rotation, the rotated right-hand side, the history and the stopping tests (one thread).
+// col, cs, sn: the Hessenberg column being formed and the rotations, in global memory or staged in
+// shared memory by the caller with col already holding h (the rotation chain is sequential; staged, each
+// step costs a shared-memory access instead of a global one). rotated: col's previous rotations are applied.
+__device__ void arnoldi_finish(GmState& S, GmArrays& ar, int rhs, double s, double2* col, double2* cs, double2* sn,
+                               bool staged, bool rotated = false) {
     const double sub = sqrt(s);
     const int m = ar.m, j = S.step;
     double2* g = ar.g + (int64_t)rhs * (m + 1);
+    const double2* h = ar.h + (int64_t)rhs * (m + 1);
+    if (!staged)
+        for (int k = 0; k <= j; ++k) col[k] = h[k];
     col[j + 1] = make_double2(sub, 0);
+    for (int k = rotated ? j : 0; k < j; ++k) {
+        const double2 a0 = col[k], a1 = col[k + 1];
+        col[k] = dadd(dmulc(cs[k], a0), dmulc(sn[k], a1));
+        const double2 t = dmul(sn[k], a0);
+        const double2 u = dmul(cs[k], a1);
+        col[k + 1] = make_double2(u.x - t.x, u.y - t.y);
+    }
     // generateRotation_.m:11-18
     const double2 a = col[j], bsub = col[j + 1];
     const double radius = sqrt(a.x * a.x + a.y * a.y + bsub.x * bsub.x + bsub.y * bsub.y);
@@ -419,26 +433,6 @@ __device__ void arnoldi_rotate(GmState& S, GmArrays& ar, int rhs, double s, doub
     S.done = S.converged || S.iteration >= S.max_iterations;
 }
 
-// The rest of an Arnoldi step once ||w|| is known: the Hessenberg column, its previous rotations,
-// the new rotation, the rotated right-hand side, the history and the stopping tests (one thread).
-// col, cs, sn: the Hessenberg column being formed and the rotations, in global memory or staged in
-// shared memory by the caller with col already holding h (the rotation chain is sequential; staged, each
-// step costs a shared-memory access instead of a global one).
-__device__ void arnoldi_finish(GmState& S, GmArrays& ar, int rhs, double s, double2* col, double2* cs, double2* sn,
-                               bool staged) {
-    const int m = ar.m, j = S.step;
-    const double2* h = ar.h + (int64_t)rhs * (m + 1);
-    if (!staged)
-        for (int k = 0; k <= j; ++k) col[k] = h[k];
-    for (int k = 0; k < j; ++k) {
-        const double2 a0 = col[k], a1 = col[k + 1];
-        col[k] = dadd(dmulc(cs[k], a0), dmulc(sn[k], a1));
-        const double2 t = dmul(sn[k], a0);
-        const double2 u = dmul(cs[k], a1);
-        col[k + 1] = make_double2(u.x - t.x, u.y - t.y);
-    }
-    arnoldi_rotate(S, ar, rhs, s, col, cs, sn);
-}
 // Asynchronous global -> shared copies (cp.async, sm_80 and later): a thread issues all the copies
 // of a tile without waiting, then waits for its groups before the CTA barrier.
 template <int BYTES> __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
@@ -1226,7 +1220,7 @@ __global__ void __launch_bounds__(kArnThreads, 1)
     __syncthreads();  // scol
     if (tid == 0) {
         S.bar_base = at;
-        arnoldi_rotate(S, ar, rhs, sub2, scol, ar.cs + (int64_t)rhs * m, ar.sn + (int64_t)rhs * m);
+        arnoldi_finish(S, ar, rhs, sub2, scol, ar.cs + (int64_t)rhs * m, ar.sn + (int64_t)rhs * m, true, true);
     }
     __syncthreads();
     double2* column = ar.H + ((int64_t)rhs * m + j) * (m + 1);
